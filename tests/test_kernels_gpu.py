@@ -113,8 +113,8 @@ def test_linear_rows_do_not_depend_on_the_batch():
     one = torch.zeros(1, 130, device=DEV)
     o.linear_simt(a[41:42].to(DEV), w.to(DEV), None, one, 1)
     assert torch.equal(one[0], full[41])
-    # steps of at most 16 rows run on a kernel of their own (a thread per feature, K in chunks of 64 asked
-    # for ahead): every output is still one accumulator in index order, so the bits are those of the tiled
+    # steps of at most 16 rows run on a kernel of their own (a thread per feature and segment of K): every
+    # output is still added up in one order that K alone sets, so the bits are those of the tiled
     # kernel; with bias, both activations and the residual sum, and sizes that no tile divides
     bias = torch.randn(130, generator=g)
     for act in (o.ACT_NONE, o.ACT_GELU_TANH, o.ACT_GELU_ERF):
@@ -126,6 +126,30 @@ def test_linear_rows_do_not_depend_on_the_batch():
                 few = base[m0:m0 + n].clone()
                 o.linear_simt(a[m0:m0 + n].to(DEV), w.to(DEV), bias.to(DEV), few, n, act, residual)
                 assert torch.equal(few, full[m0:m0 + n]), (act, residual, m0, n)
+
+
+@pytest.mark.parametrize("N, K", [(1, 1), (9, 31), (65, 33), (130, 260), (72, 1024), (2400, 96), (40, 1100), (24, 3076), (9600, 40)])
+@pytest.mark.parametrize("pad", [0, 1])
+def test_linear_in_32_bits_at_the_edges_of_segments_stages_and_tiles(N, K, pad):
+    """Rows around every change of kernel and tile, K around a segment (32) and a stage (1,024) of it, outputs narrow
+    enough for a split of K and wide enough to be walked; ``pad``: pitches that no 16-byte copy takes.  An output is
+    at most 32 roundings of a chain, those of a quarter's segments and a few more off (times the sum of magnitudes)."""
+    g = gen(5)
+    o = ops()
+    w = torch.randn(N, K + pad, generator=g)[:, :K].to(DEV)
+    a = torch.randn(161, K + pad, generator=g)[:, :K].to(DEV)
+    bias = torch.randn(N, generator=g).to(DEV)
+    a64, w64 = a.double(), w.double()
+    bound = (32 + K // 128 + 8) * 2.0 ** -24 * (a64.abs() @ w64.abs().T + bias.double().abs())
+    want = a64 @ w64.T + bias.double()
+    last = None
+    for M in (1, 2, 3, 4, 8, 9, 16, 17, 32, 33, 64, 65, 96, 97, 161):
+        out = torch.full((M + 1, N), 7.0, device=DEV)
+        o.linear_simt(a, w, bias, out, M)
+        assert bool(((out[:M].double() - want[:M]).abs() <= bound[:M]).all()), M
+        assert bool((out[M:] == 7.0).all())
+        assert last is None or torch.equal(out[:last.shape[0]], last), M     # whatever the other rows
+        last = out[:M].clone()
 
 
 def paged_case(dtype, n_head, n_kv_head, hd, page_size, lengths, q_lens, seed):
