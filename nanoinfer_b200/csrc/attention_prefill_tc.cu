@@ -1,21 +1,25 @@
 // Causal attention for prompt portions on the fifth-generation tensor cores: S = Q K^T and O += P V
 // by tcgen05.mma with S and O in tensor memory, keys and values brought page by page by TMA.
 //
-// One block takes 128 consecutive query rows of one request and one head (head size 64) and walks
-// the keys in tiles of 128.  Warps 0 and 6 are the TMA producers of keys and of values: their lanes
-// look the tile's pages up in the request's block table and load them (16 rows x 128 bytes a load)
-// into rings of three stages of 128-byte-swizzled shared memory.  Warp 1 issues the MMAs: S = Q K^T (128 x 128 x 64) into
-// one of three score buffers in tensor memory, three tiles ahead of the softmax; and, once the softmax
-// warps have laid P down in shared memory as bfloat16 (three buffers), O += P V (128 x 64 x 128; V is
-// read as it lies, keys down the rows, as an MN-major operand), accumulated in tensor memory over
-// all tiles.  Warps 2..5 are the softmax: a thread owns a row, so the row maximum and sum need no
-// exchange between threads.  The running maximum is only raised when a tile exceeds it by more than
-// 2^8 (P stays below 2^8, the final division by the sum is exact all the same): only then is O read
-// from tensor memory, scaled and written back, which is rare after the first tiles, so the softmax
-// warps normally go from one tile's scores to the next without waiting for an MMA.  Softmax in
-// 32-bit with scores kept times log2(e); formula and masking as in attention_prefill.cu
-// (crates/core/src/kernels/reference.rs:109-142); tiling after the reference's attn_prefill_flash
-// (crates/metal/src/shaders/attn.metal:100-218).
+// One block takes 128 consecutive query rows of one request and one head (head size 64) and walks the keys in tiles of
+// 128; two blocks share an SM.  Warp 0 is the TMA producer: its lanes look the tile's pages up in the request's block
+// table and load them (16 rows x 128 bytes a load; lanes 0..7 keys, lanes 8..15 values) into rings of two stages of
+// 128-byte-swizzled shared memory.  Warp 1 issues the MMAs: S = Q K^T (128 x 128 x 64) into tensor memory, the next
+// tile's as soon as the softmax warps hold this one's scores in registers; and, once they have written P to tensor
+// memory as bfloat16, O += P V (128 x 64 x 128, P the operand that tensor memory holds, V read as it lies, keys down
+// the rows, as an MN-major operand).  Warps 2..5 are the softmax: a thread owns a row, so the row maximum and sum need
+// no exchange between threads.  The running maximum is only raised when a tile exceeds it by more than 2^8 (P stays
+// below 2^8, the final division by the sum is exact all the same): only then is O read from tensor memory, scaled and
+// written back, which is rare after the first tiles.  Softmax in 32-bit with scores kept times log2(e), products and
+// sums two at a time; formula and masking as in attention_prefill.cu (crates/core/src/kernels/reference.rs:109-142);
+// tiling after the reference's attn_prefill_flash (crates/metal/src/shaders/attn.metal:100-218).
+//
+// What bounds it: the 128 x 128 exponentials of a tile take an SM 1,024 cycles, everything else of a softmax warp about
+// 500 issue slots; one warp a scheduler does these one after another, and with the start and end of a block in the
+// open.  With one block an SM (P through shared memory, scores three tiles ahead) a tile took 2,800 cycles; two blocks
+// an SM, each half as deep, fill each other's waits: 1,750.  On a B200, us before and now: 8 prompts of 1,003 rows and
+// 25 heads 120, 72; one of 8,144 rows and 12 heads 248, 156 (411, 655 TFLOP/s; the unit that makes the
+// exponentials 63 % busy); 2 x 1,024 rows and 12 heads, where a block has an SM to itself, 17.5, 18.0.
 //
 // With EX the kernel takes the options of AttnExtras (api.h).  The softmax threads bring every score to its final
 // form first (scale, cap, distance bias, times log2(e); the cap by tanh(x) = 1 - 2 / (1 + e^2x) with the hardware's
@@ -33,7 +37,8 @@ namespace nib {
 
 constexpr int AT_BM = 128;      // query rows per block = MMA M
 constexpr int AT_HD = 64;       // head size: one 128-byte swizzle row
-constexpr int AT_THREADS = 224;   // keys' producer, MMA issue, four softmax warps, values' producer
+constexpr int AT_THREADS = 192;   // producer, MMA issue, four softmax warps
+constexpr int AT_BN = 128;        // keys per tile
 constexpr int AT_UNIT = 16;     // rows of one TMA load of keys or values (divides the page size)
 
 struct AtParams {
@@ -92,43 +97,86 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-constexpr int AT_STAGES = 3;     // stages of keys and values
-constexpr int AT_NBUF = 3;       // score buffers in tensor memory and P buffers in shared memory
+// 32 columns of tensor memory on their way to registers, and, after tmem_ld_wait(), the place from which on they may be used
+__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, float* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+        "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]),
+        "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]),
+        "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld32_ready(float* v) {
+  asm volatile("" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]),
+        "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]), "+f"(v[16]),
+        "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]), "+f"(v[23]), "+f"(v[24]),
+        "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]), "+f"(v[29]));
+  asm volatile("" : "+f"(v[30]), "+f"(v[31]));
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+// D (+)= A B with A (128 rows, 16 values of K: eight columns of pairs) in tensor memory
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// two 32-bit products or sums in one instruction (each rounded as its own)
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void f32x2_split(uint64_t d, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(d));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+constexpr int AT_STAGES = 2;     // stages of keys and of values
+constexpr int AT_KV_STAGE = AT_BN * 128;   // bytes of a stage: [128 keys][64]
+// tensor memory: scores (128 columns), P (64 columns of pairs), O (64)
+constexpr uint32_t AT_P_COL = AT_BN, AT_O_COL = AT_BN + AT_BN / 2, AT_TMEM_COLS = 256;
+constexpr size_t AT_SMEM = 16384 + 2 * AT_STAGES * AT_KV_STAGE + 1024;
 constexpr float AT_RAISE = 8.0f; // the running maximum is raised when a tile exceeds it by more than 2^8
 
-// AT_BN: keys per tile.  64: two blocks an SM (256 columns of tensor memory and 97 KB each); 128: one
-// block an SM with the whole tensor memory, half as many MMA instructions per key for the scores (an
-// instruction of this shape takes about 128 cycles however narrow it is).
-template <int AT_BN>
-struct AtShape {
-  static constexpr int KV_STAGE = AT_BN * 128;            // bytes of a stage of keys (or values): [BN keys][64]
-  static constexpr int P_BYTES = (AT_BN / 64) * 16384;    // one P buffer: [BN / 64 key blocks][128 rows][64 keys]
-  static constexpr uint32_t O_COL = AT_NBUF * AT_BN;      // tensor memory: the score buffers, then O
-  static constexpr uint32_t TMEM_COLS = AT_BN == 64 ? 256 : 512;
-  static constexpr size_t SMEM = 16384 + 2 * AT_STAGES * KV_STAGE + AT_NBUF * P_BYTES + 1024;
-};
-
-template <int AT_BN, bool EX>
-__global__ void __launch_bounds__(AT_THREADS, AT_BN == 64 ? 2 : 1)
+template <bool EX>
+__global__ void __launch_bounds__(AT_THREADS, 2)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                             const AtParams prm) {
   pdl_trigger();
   extern __shared__ uint8_t at_smem_raw[];
   // tiles must start on a 1024-byte boundary for the 128-byte swizzle
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)at_smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr int AT_KV_STAGE = AtShape<AT_BN>::KV_STAGE, P_BYTES = AtShape<AT_BN>::P_BYTES;
-  constexpr uint32_t O_COL = AtShape<AT_BN>::O_COL, TMEM_COLS = AtShape<AT_BN>::TMEM_COLS;
   uint8_t* q_s = smem;                                  // [128 rows][64]              16 KB
-  uint8_t* k_s = q_s + 16384;                           // [stages][BN keys][64]
-  uint8_t* v_s = k_s + AT_STAGES * AT_KV_STAGE;         // [stages][BN keys][64]
-  uint8_t* p_s = v_s + AT_STAGES * AT_KV_STAGE;         // [2][BN / 64][128 rows][64 keys]
+  uint8_t* k_s = q_s + 16384;                           // [stages][128 keys][64]
+  uint8_t* v_s = k_s + AT_STAGES * AT_KV_STAGE;         // [stages][128 keys][64]
   __shared__ __align__(8) uint64_t q_full, k_full[AT_STAGES], k_empty[AT_STAGES], v_full[AT_STAGES], v_empty[AT_STAGES],
-      s_full[AT_NBUF], p_full[AT_NBUF], o_full[AT_NBUF];
+      s_full, s_empty, p_full, o_full;
   __shared__ uint32_t tmem_base_sh;
   __shared__ int abort_sh;
   volatile int* abort_flag = &abort_sh;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   // (heads are the fast index of the grid: blocks start in the order of the tile list, longest first)
   const int e = prm.tiles[2 * blockIdx.y], q_off = prm.tiles[2 * blockIdx.y + 1];
   const int h = blockIdx.x, hk = h / (prm.n_head / prm.n_kv_head);
@@ -157,32 +205,27 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 1);
     }
-    for (int i = 0; i < AT_NBUF; ++i) {
-      mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], 128);
-      mbar_init(&o_full[i], 1);
-    }
+    mbar_init(&s_full, 1);
+    mbar_init(&s_empty, 128);
+    mbar_init(&p_full, 128);
+    mbar_init(&o_full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // tensor memory: the score buffers (BN columns each), then the output O (64 columns)
-  if (warp == 1) tmem_alloc(&tmem_base_sh, TMEM_COLS);
+  if (warp == 1) tmem_alloc(&tmem_base_sh, AT_TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_base_sh;
-  pdl_wait();   // the queries, and this step's keys and values, come from the kernels ahead
+  const uint32_t tmem_base = warp_uniform(tmem_base_sh);
+  if (warp != 0) pdl_wait();   // the queries, and this step's keys and values, come from the kernels ahead
 
-  if (warp == 0 || warp == 6) {
-    // ---------------- producers: Q once, then a stage of keys (warp 0) and of values (warp 6) per
-    // tile.  A load brings one unit of 16 rows; lane u issues unit u of its tile, with its own look-up
-    // in the block table, so a tile's loads leave together.
-    const bool is_v = warp == 6;
-    if (!is_v && lane == 0) {
-      mbar_expect_tx(&q_full, 16384);
-      tma_load_2d(q_s, &map_q, &q_full, h * AT_HD, row0);
-    }
-    const int u = lane;
-    const bool active = u < AT_BN / AT_UNIT;
+  if (warp == 0) {
+    // ---------------- producer: Q once, then a stage of keys and one of values per tile.  A load brings one unit of 16
+    // rows; lane u issues unit u % 8 of its tile, with its own look-up in the block table, so a tile's loads leave
+    // together.
+    constexpr int UNITS = AT_BN / AT_UNIT;
+    const bool is_v = lane >= UNITS;
+    const int u = lane % UNITS;
+    const bool active = lane < 2 * UNITS;
     bool ok = true;
     // keys outside [key_lo, pos_last] are masked; their rows are read from the nearest unit of the
     // request that is there (finite values, weight zero)
@@ -198,65 +241,74 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       }
       return ((page * 2) * prm.n_kv_head + hk) * prm.page_size + j % prm.page_size;
     };
-    // The two warps run loops of their own: the keys' warp is held back only by the scores (a stage's
-    // keys are free as soon as the scores are made from them), the values' warp by the P V products,
-    // so the keys that the scores three tiles ahead wait for leave early.
     uint8_t* dst_base = (is_v ? v_s : k_s) + u * 2048;
     const int row_off = is_v ? prm.n_kv_head * prm.page_size : 0;
-    int row_next = unit_row(0);
+    int row_next = unit_row(0);      // (the step's tables were there before the kernel ahead)
+    pdl_wait();
+    if (lane == 0) {
+      mbar_expect_tx(&q_full, 16384);
+      tma_load_2d(q_s, &map_q, &q_full, h * AT_HD, row0);
+    }
     for (int it = 0; it < n_it; ++it) {
       const int st = it % AT_STAGES, round = it / AT_STAGES;
       const int row = row_next;
-      row_next = unit_row(it + 1);   // the next tile's look-up travels while this tile's stage is waited for
-      uint64_t* empty = is_v ? &v_empty[st] : &k_empty[st];
-      uint64_t* full = is_v ? &v_full[st] : &k_full[st];
-      if (round > 0) ok = warp_mbar_wait(empty, (round + 1) & 1, abort_flag, lane);
+      row_next = unit_row(it + 1);   // the next tile's look-up travels while this tile's stages are waited for
+      // the keys' stage is free once the scores are made from it, which is before the values' is
+      if (round > 0) ok = warp_mbar_wait(&k_empty[st], (round + 1) & 1, abort_flag, lane);
       if (!ok) break;
-      if (lane == 0) mbar_expect_tx(full, AT_KV_STAGE);
+      if (lane == 0) mbar_expect_tx(&k_full[st], AT_KV_STAGE);
       __syncwarp();
-      if (active) tma_load_2d(dst_base + st * AT_KV_STAGE, &map_kv, full, 0, row + row_off);
+      if (active && !is_v) tma_load_2d(dst_base + st * AT_KV_STAGE, &map_kv, &k_full[st], 0, row);
+      if (round > 0) ok = warp_mbar_wait(&v_empty[st], (round + 1) & 1, abort_flag, lane);
+      if (!ok) break;
+      if (lane == 0) mbar_expect_tx(&v_full[st], AT_KV_STAGE);
+      __syncwarp();
+      if (active && is_v) tma_load_2d(dst_base + st * AT_KV_STAGE, &map_kv, &v_full[st], 0, row + row_off);
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issue
-    if (lane == 0) {
-      const uint32_t idesc_s = umma_idesc(AT_BM, AT_BN);
-      const uint32_t idesc_o = umma_idesc(AT_BM, AT_HD) | (1u << 16);   // B (= V) is MN-major: keys down the rows
-      const uint32_t o_tmem = tmem_base + O_COL;
-      // scores of tile `it` into buffer it % AT_NBUF (free: P of tile it - AT_NBUF was made from it)
-      auto issue_s = [&](int it) -> bool {
-        const int st = it % AT_STAGES;
-        if (!mbar_wait(&k_full[st], (it / AT_STAGES) & 1, abort_flag)) return false;
-        tc_fence_after();
-        const uint32_t qa = smem_u32(q_s), kb = smem_u32(k_s + st * AT_KV_STAGE);
+    // ---------------- MMA issue: the whole warp walks, one lane issues
+    const bool leader = elect_one();
+    const uint32_t idesc_s = umma_idesc(AT_BM, AT_BN);
+    const uint32_t idesc_o = umma_idesc(AT_BM, AT_HD) | (1u << 16);   // B (= V) is MN-major: keys down the rows
+    const uint32_t o_tmem = tmem_base + AT_O_COL, p_tmem = tmem_base + AT_P_COL;
+    const uint32_t q_lo = umma_desc_lo(smem_u32(q_s)), k_lo = umma_desc_lo(smem_u32(k_s)), v_lo = umma_desc_lo(smem_u32(v_s));
+    auto issue_s = [&](int it) -> bool {
+      const int st = it % AT_STAGES;
+      if (!warp_mbar_wait(&k_full[st], (it / AT_STAGES) & 1, abort_flag, lane)) return false;
+      tc_fence_after();
+      if (leader) {
 #pragma unroll
         for (int k = 0; k < AT_HD / 16; ++k)   // 16 of the head's 64 values per instruction: 32 bytes along the row
-          umma_bf16(tmem_base + (uint32_t)((it % AT_NBUF) * AT_BN), umma_desc(qa + k * 32), umma_desc(kb + k * 32),
-                    idesc_s, k > 0);
-        umma_commit(&s_full[it % AT_NBUF]);
+          umma_bf16(tmem_base, umma_desc_of(q_lo + 2 * k), umma_desc_of(k_lo + st * (AT_KV_STAGE / 16) + 2 * k), idesc_s, k > 0);
+        umma_commit(&s_full);
         umma_commit(&k_empty[st]);
-        return true;
-      };
-      bool ok = mbar_wait(&q_full, 0, abort_flag);
-      if (ok) ok = issue_s(0);
-      for (int a = 1; ok && a < AT_NBUF && a < n_it; ++a) ok = issue_s(a);
-      for (int it = 0; ok && it < n_it; ++it) {
-        const int st = it % AT_STAGES, b = it % AT_NBUF;
-        if (!mbar_wait(&v_full[st], (it / AT_STAGES) & 1, abort_flag)) break;
-        if (!mbar_wait(&p_full[b], (it / AT_NBUF) & 1, abort_flag)) break;
-        tc_fence_after();
-        const uint32_t vb = smem_u32(v_s + st * AT_KV_STAGE);
-        const uint32_t pa = smem_u32(p_s + b * P_BYTES);
-#pragma unroll
-        for (int k = 0; k < AT_BN / 16; ++k)   // 16 keys per instruction: P 32 bytes along its row, V 16 rows down
-          umma_bf16(o_tmem, umma_desc(pa + (k >> 2) * 16384 + (k & 3) * 32), umma_desc(vb + k * 2048), idesc_o,
-                    (it > 0 || k > 0) ? 1u : 0u);
-        umma_commit(&o_full[b]);
-        umma_commit(&v_empty[st]);
-        if (it + AT_NBUF < n_it) ok = issue_s(it + AT_NBUF);
       }
+      __syncwarp();
+      return true;
+    };
+    bool ok = warp_mbar_wait(&q_full, 0, abort_flag, lane);
+    if (ok) ok = issue_s(0);
+    for (int it = 0; ok && it < n_it; ++it) {
+      const int st = it % AT_STAGES;
+      if (it + 1 < n_it) {
+        if (!warp_mbar_wait(&s_empty, it & 1, abort_flag, lane)) break;   // the scores are in the softmax threads' registers
+        tc_fence_after();
+        if (!issue_s(it + 1)) break;
+      }
+      if (!warp_mbar_wait(&v_full[st], (it / AT_STAGES) & 1, abort_flag, lane)) break;
+      if (!warp_mbar_wait(&p_full, it & 1, abort_flag, lane)) break;
+      tc_fence_after();
+      if (leader) {
+#pragma unroll
+        for (int k = 0; k < AT_BN / 16; ++k)   // 16 keys per instruction: eight columns of P, V 16 rows down
+          umma_bf16_ts(o_tmem, p_tmem + k * 8, umma_desc_of(v_lo + st * (AT_KV_STAGE / 16) + k * 128), idesc_o,
+                       (it > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&o_full);
+        umma_commit(&v_empty[st]);
+      }
+      __syncwarp();
     }
-    __syncwarp();
   } else {
     // ---------------- softmax: a thread per row; warp w owns tensor-memory lanes 32 * (w % 4) .. +32
     const int quarter = warp & 3;
@@ -276,8 +328,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     float m = -INFINITY, l = 0.0f;
     bool ok = true;
     for (int it = 0; it < n_it; ++it) {
-      const int b = it % AT_NBUF;
-      ok = warp_mbar_wait(&s_full[b], (it / AT_NBUF) & 1, abort_flag, lane);
+      ok = warp_mbar_wait(&s_full, it & 1, abort_flag, lane);
       if (!ok) break;
       tc_fence_after();
       const int j0 = tile_of(it) * AT_BN;
@@ -285,7 +336,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                         (span > 0 && j0 < wp1 - wp1 % span);   // only these tiles need the mask
       float v[AT_BN];
 #pragma unroll
-      for (int c = 0; c < AT_BN / 32; ++c) tmem_ld32(lane_addr + (uint32_t)(b * AT_BN + c * 32), v + c * 32);
+      for (int c = 0; c < AT_BN / 32; ++c) tmem_ld32_issue(lane_addr + (uint32_t)(c * 32), v + c * 32);
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < AT_BN / 32; ++c) tmem_ld32_ready(v + c * 32);
+      tc_fence_before();
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&s_empty)) : "memory");
       if (EX) {
         const float far = (float)(p - j0);
         if (cap_in > 0.0f) {
@@ -321,48 +377,56 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           const float corr = (m_new == -INFINITY) ? 1.0f : at_pow2(m - m_new);
           l *= corr;
           // O holds the tiles up to it - 1 once their MMAs are done
-          ok = warp_mbar_wait(&o_full[(it - 1) % AT_NBUF], ((it - 1) / AT_NBUF) & 1, abort_flag, lane);
+          ok = warp_mbar_wait(&o_full, (it - 1) & 1, abort_flag, lane);
           if (!ok) break;
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < AT_HD / 32; ++c) {
             float t[32];
-            tmem_ld32(lane_addr + O_COL + (uint32_t)(c * 32), t);
+            tmem_ld32(lane_addr + AT_O_COL + (uint32_t)(c * 32), t);
 #pragma unroll
             for (int i = 0; i < 32; ++i) t[i] *= corr;
-            tmem_st32(lane_addr + O_COL + (uint32_t)(c * 32), t);
+            tmem_st32(lane_addr + AT_O_COL + (uint32_t)(c * 32), t);
           }
         }
         m = m_new;
       }
       // a row with no key yet (all masked so far) keeps m = -inf; 2^(-inf - -inf) is avoided
       const float ms = (m == -INFINITY) ? 0.0f : m;
-      // P of tile it - AT_NBUF (the last user of this buffer) has been read by its MMA
-      if (it >= AT_NBUF) {
-        ok = warp_mbar_wait(&o_full[b], ((it - AT_NBUF) / AT_NBUF) & 1, abort_flag, lane);
+      // P of the tile before has been read by its MMA
+      if (it > 0) {
+        ok = warp_mbar_wait(&o_full, (it - 1) & 1, abort_flag, lane);
         if (!ok) break;
+        tc_fence_after();
       }
-      float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      uint8_t* blk0 = p_s + b * P_BYTES + r * 128;
+      uint64_t sum_a = 0, sum_b = 0;    // (pairs of zeros) four chains
+      const uint64_t scale_2 = f32x2(scale2, scale2), less_2 = f32x2(-ms, -ms);
 #pragma unroll
-      for (int g = 0; g < AT_BN / 8; ++g) {
-        uint8_t* blk = blk0 + (g >> 3) * 16384;   // 64 keys (eight 16-byte pieces) a block
-        float e8[8];
+      for (int c = 0; c < AT_BN / 32; ++c) {
+        uint32_t pk[16];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          e8[i] = at_pow2(fmaf(v[8 * g + i], scale2, -ms));   // 0 for a masked key
-          sum4[i & 3] += e8[i];
+        for (int i = 0; i < 16; i += 2) {
+          float e0, e1, e2, e3;
+          f32x2_split(fma_f32x2(f32x2(v[c * 32 + 2 * i], v[c * 32 + 2 * i + 1]), scale_2, less_2), e0, e1);
+          f32x2_split(fma_f32x2(f32x2(v[c * 32 + 2 * i + 2], v[c * 32 + 2 * i + 3]), scale_2, less_2), e2, e3);
+          e0 = at_pow2(e0); e1 = at_pow2(e1); e2 = at_pow2(e2); e3 = at_pow2(e3);   // 0 for a masked key
+          sum_a = add_f32x2(sum_a, f32x2(e0, e1));
+          sum_b = add_f32x2(sum_b, f32x2(e2, e3));
+          pk[i] = pack_bf16(e0, e1);
+          pk[i + 1] = pack_bf16(e2, e3);
         }
-        *reinterpret_cast<uint4*>(blk + (((g & 7) ^ (r & 7)) * 16)) =
-            make_uint4(pack_bf16(e8[0], e8[1]), pack_bf16(e8[2], e8[3]), pack_bf16(e8[4], e8[5]), pack_bf16(e8[6], e8[7]));
+        tmem_st16(lane_addr + AT_P_COL + (uint32_t)(c * 16), pk);
       }
-      l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the MMAs
+      float s0, s1, s2, s3;
+      f32x2_split(sum_a, s0, s1);
+      f32x2_split(sum_b, s2, s3);
+      l += (s0 + s1) + (s2 + s3);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&p_full[b])) : "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&p_full)) : "memory");
     }
     // the last MMA into O
-    if (ok) ok = warp_mbar_wait(&o_full[(n_it - 1) % AT_NBUF], ((n_it - 1) / AT_NBUF) & 1, abort_flag, lane);
+    if (ok) ok = warp_mbar_wait(&o_full, (n_it - 1) & 1, abort_flag, lane);
     if (ok) {
       tc_fence_after();
       // (the sink's term is exp(0) unless the heads have logits of their own)
@@ -376,7 +440,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll 1
       for (int c = 0; c < AT_HD / 32; ++c) {
         float t[32];
-        tmem_ld32(lane_addr + O_COL + (uint32_t)(c * 32), t);
+        tmem_ld32(lane_addr + AT_O_COL + (uint32_t)(c * 32), t);
         if (EX && prm.ex.out32) {
           float* dst32 = reinterpret_cast<float*>(prm.out) + (size_t)(row0 + r) * prm.ldo + h * AT_HD;
           if (r < n_rows) {
@@ -400,7 +464,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   if (threadIdx.x == 0 && abort_sh) *prm.status = NIB_STATUS_WAIT_TIMEOUT;
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    tmem_dealloc(tmem_base, AT_TMEM_COLS);
   }
 }
 
@@ -444,23 +508,20 @@ extern "C" int nib_attention_prefill_tc(const void* q, int ldq, int T, const voi
   prm.n_head = n_head; prm.n_kv_head = n_kv_head; prm.page_size = page_size; prm.n_pages = n_pages;
   prm.scale = scale; prm.window = window; prm.sink = sink; prm.out = (bf16*)out; prm.ldo = ldo; prm.status = status;
   prm.ex = AttnExtras{softcap, keep_first, slopes, gate, ldg, out_scale, span, head_scale, sinks, out32, gate_dim, pool, pool_table};
-  // 128 keys a tile, one block an SM: measured a little faster than 64 keys a tile and two blocks
-  constexpr int BN = 128;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)AtShape<BN>::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)AT_SMEM);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attention_prefill_tc_kernel<BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)AtShape<BN>::SMEM);
+      e = cudaFuncSetAttribute(attention_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
   if (plain)
-    launch_pdl(attention_prefill_tc_kernel<BN, false>, dim3(n_head, n_tiles), dim3(AT_THREADS), AtShape<BN>::SMEM, stream,
+    launch_pdl(attention_prefill_tc_kernel<false>, dim3(n_head, n_tiles), dim3(AT_THREADS), AT_SMEM, stream,
                map_q, map_kv, prm);
   else
-    launch_pdl(attention_prefill_tc_kernel<BN, true>, dim3(n_head, n_tiles), dim3(AT_THREADS), AtShape<BN>::SMEM, stream,
+    launch_pdl(attention_prefill_tc_kernel<true>, dim3(n_head, n_tiles), dim3(AT_THREADS), AT_SMEM, stream,
                map_q, map_kv, prm);
   NIB_LAUNCH_CHECK();
 }

@@ -114,6 +114,27 @@ __device__ __forceinline__ uint32_t umma_idesc(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// The descriptor of the low half `lo` (umma_desc_lo of a tile, plus 16-byte units along it): the high half is the same
+// for every tile.
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr) { return (uint32_t)umma_desc(smem_addr); }
+__device__ __forceinline__ uint64_t umma_desc_of(uint32_t lo) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"((uint32_t)(umma_desc(0) >> 32)));
+  return d;
+}
+
+// One lane of a converged warp.  The tensor-core and TMA instructions take their operands from registers that a whole
+// warp shares.  Issued under a condition on the thread (`lane == 0`) each operand has to be gathered from the one
+// thread that is active, about 100 cycles an instruction on a B200; in code that the whole warp runs, on values that
+// are the same in all lanes (`warp_uniform`), with this one lane issuing, an MMA of 128 x 64 x 16 takes 32 to 48
+// cycles and one of 128 x 256 x 16 takes 129 instead of 172: what the tensor cores take.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.b32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
+}
+template <typename T> __device__ __forceinline__ T warp_uniform(T v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&h);
