@@ -129,7 +129,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   __shared__ int abort_sh;
   volatile int* abort_flag = &abort_sh;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   // (heads are the fast index of the grid: blocks start in the order of the tile list, longest first)
   const int e = prm.tiles[2 * blockIdx.y], q_off = prm.tiles[2 * blockIdx.y + 1];
   const int row0 = prm.entry_start[e] + q_off;                    // first row of the tile in the step
@@ -166,7 +166,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   __syncthreads();
   pdl_trigger();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_base_sh;
+  const uint32_t tmem_base = warp_uniform(tmem_base_sh);
 
   if (warp == 0) {
     // ---------------- producer
@@ -210,55 +210,65 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issue
-    if (lane == 0) {
-      const uint32_t idesc_s = umma_idesc(LP_BM, LP_BN);
-      const uint32_t idesc_o = umma_idesc(LP_BM, nv * 64) | (1u << 16);   // B (= V) is MN-major: keys down the rows
-      const uint32_t o_tmem = tmem_base + LP_O_COL;
-      const uint32_t qa = smem_u32(q_s);
-      auto issue_s = [&](int it) {
-        tc_fence_after();
-        const uint32_t kb = smem_u32(k_s + (it % stages) * stage_bytes);
+    // ---------------- MMA issue: the whole warp walks, one lane issues
+    const bool leader = elect_one();
+    const uint32_t idesc_s = umma_idesc(LP_BM, LP_BN);
+    const uint32_t idesc_o = umma_idesc(LP_BM, nv * 64) | (1u << 16);   // B (= V) is MN-major: keys down the rows
+    const uint32_t o_tmem = tmem_base + LP_O_COL;
+    const uint32_t q_lo = umma_desc_lo(smem_u32(q_s)), k_lo = umma_desc_lo(smem_u32(k_s)), p_lo = umma_desc_lo(smem_u32(p_s));
+    // (V's chunks lie LP_CHUNK_K bytes apart along the values: that is the descriptor's leading byte offset)
+    const uint32_t v_lo = (umma_desc_lo(smem_u32(k_s + v_off)) & ~(0x3fffu << 16)) | ((uint32_t)(LP_CHUNK_K >> 4) << 16);
+    auto issue_s = [&](int it) {
+      tc_fence_after();
+      if (leader) {
+        const uint32_t kt = k_lo + (uint32_t)(it % stages) * (uint32_t)(stage_bytes >> 4);
         for (int ks = ks_lo; ks < ks_hi; ++ks) {   // 16 values per instruction: 32 bytes along a chunk's row
           const int c = ks / 4 - c_lo, k = ks & 3;
-          umma_bf16(tmem_base + (uint32_t)((it % LP_NBUF) * LP_BN), umma_desc(qa + c * LP_CHUNK_Q + k * 32),
-                    umma_desc(kb + c * LP_CHUNK_K + k * 32), idesc_s, ks > ks_lo ? 1u : 0u);
+          umma_bf16(tmem_base + (uint32_t)((it % LP_NBUF) * LP_BN), umma_desc_of(q_lo + c * (LP_CHUNK_Q >> 4) + k * 2),
+                    umma_desc_of(kt + c * (LP_CHUNK_K >> 4) + k * 2), idesc_s, ks > ks_lo ? 1u : 0u);
         }
         umma_commit(&s_full[it % LP_NBUF]);
-      };
-      // (V's chunks lie LP_CHUNK_K bytes apart along the values: that is the descriptor's leading byte offset)
-      const uint64_t lead = (uint64_t)(LP_CHUNK_K >> 4) << 16;
-      auto v_desc = [&](uint32_t addr) { return (umma_desc(addr) & ~(0x3fffull << 16)) | lead; };
-      auto issue_pv = [&](int it) {
-        tc_fence_after();
+      }
+      __syncwarp();
+    };
+    auto issue_pv = [&](int it) {
+      tc_fence_after();
+      if (leader) {
         const int st = it % stages, b = it % LP_NBUF;
-        const uint32_t vb = smem_u32(k_s + st * stage_bytes + v_off), pa = smem_u32(p_s + b * LP_P_BYTES);
+        const uint32_t vt = v_lo + (uint32_t)st * (uint32_t)(stage_bytes >> 4), pt = p_lo + (uint32_t)b * (LP_P_BYTES >> 4);
 #pragma unroll
         for (int k = 0; k < LP_BN / 16; ++k)   // 16 keys per instruction: P 32 bytes along its row, V 16 rows down
-          umma_bf16(o_tmem, umma_desc(pa + k * 32), v_desc(vb + k * 2048), idesc_o, (it > 0 || k > 0) ? 1u : 0u);
+          umma_bf16(o_tmem, umma_desc_of(pt + k * 2), umma_desc_of(vt + k * 128), idesc_o, (it > 0 || k > 0) ? 1u : 0u);
         umma_commit(&o_full[b]);
         umma_commit(&k_empty[st]);
-      };
-      bool ok = mbar_wait(&q_full, 0, abort_flag);
-      int s_next = 0, pv_next = 0;
-      long long t0 = clock64();
-      while (ok && pv_next < n_it) {
+      }
+      __syncwarp();
+    };
+    bool ok = warp_mbar_wait(&q_full, 0, abort_flag, lane);
+    int s_next = 0, pv_next = 0;
+    long long t0 = clock64();
+    enum { NOTHING, PV, SCORES, GIVE_UP };
+    while (ok && pv_next < n_it) {
+      int next = NOTHING;              // (one lane looks, for the whole warp)
+      if (lane == 0) {
         if (pv_next < s_next && lp_test(&p_full[pv_next % LP_NBUF], (pv_next / LP_NBUF) & 1)) {
-          issue_pv(pv_next++);
-          t0 = clock64();
+          next = PV;
         } else if (s_next < n_it && s_next < pv_next + LP_NBUF && lp_test(&k_full[s_next % stages], (s_next / stages) & 1)) {
           // (the score buffer is free: P of two tiles ago was made from it, or its P V would not have been issued)
-          issue_s(s_next++);
-          t0 = clock64();
+          next = SCORES;
         } else if (*abort_flag) {
-          ok = false;
+          next = GIVE_UP;
         } else if (clock64() - t0 > TC_WAIT_CYCLES) {
           *abort_flag = 1;
-          ok = false;
+          next = GIVE_UP;
         }
       }
+      next = warp_uniform(next);
+      if (next == PV) issue_pv(pv_next++);
+      else if (next == SCORES) issue_s(s_next++);
+      else if (next == GIVE_UP) ok = false;
+      if (next != NOTHING) t0 = clock64();
     }
-    __syncwarp();
   } else {
     // ---------------- softmax: a thread per row; warp w owns tensor-memory lanes 32 * (w % 4) .. +32
     const int quarter = warp & 3;

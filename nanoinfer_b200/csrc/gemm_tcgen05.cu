@@ -116,7 +116,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
   __shared__ __align__(16) float bias_sh[256];   // the bias of the tile's columns (plain orientation)
   __shared__ int fix_last_sh;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int stages = prm.stages, bq = prm.bq;
   const int k_sub = prm.k_sub;
   const bool ln = prm.ln_x != nullptr;            // the Q operand is made here, not loaded
@@ -151,18 +151,15 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_base_sh;
+  const uint32_t tmem_base = warp_uniform(tmem_base_sh);
   volatile int* abort_flag = &abort_sh;
   // Only the producer goes on before the kernel ahead has finished: it asks for the WEIGHT tiles of
   // the first stages (they do not depend on that kernel), and waits before it asks for activations.
   if (warp != 0) pdl_wait();
 
   if (warp == 0) {
-    // ---------------- TMA producer.  Issuing a stage costs one thread several hundred cycles (a wait,
-    // an expect and the copies, each a dependent instruction), so up to four lanes issue in
-    // parallel: lane l takes the stage steps l, l + L, ... (the same instructions on different
-    // barriers and buffers, so the lanes run in lockstep).
-    const int L = stages < 4 ? stages : 4;
+    // ---------------- TMA producer: the warp walks, one lane issues
+    const bool leader = elect_one();
     const bool weights_are_p = prm.swap != 0;
     // a tile of the N side; with segments, block kx of K is block kx % seg_k of segment kx / seg_k (past the end of K stays
     // past the end: zeros)
@@ -172,47 +169,54 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
     };
     // first round (the stages are all free): the weight tiles now, the activation tiles after the wait
     const int first_round = num_kb < stages ? num_kb : stages;
-    if (lane < L) {
-      for (int kb = lane; kb < first_round; kb += L) {
+    // the column of K where 64-wide block `sub` of stage step kb begins (a block past this split's end is asked for past
+    // the end of K: it arrives as zeros)
+    auto k_of = [&](int kb, int sub) {
+      const int kb64 = kb_begin + kb * k_sub + sub;
+      return (kb64 < kb_end ? kb64 : (prm.K + TC_BK - 1) / TC_BK) * TC_BK;
+    };
+    for (int kb = 0; kb < first_round; ++kb) {
+      if (leader) {
         uint8_t* sp = smem + (size_t)kb * stage_bytes;
         mbar_expect_tx(&full_bar[kb], stage_bytes);
         for (int sub = 0; sub < k_sub; ++sub) {
-          const int kb64 = kb_begin + kb * k_sub + sub;
-          const int kx = (kb64 < kb_end ? kb64 : (prm.K + TC_BK - 1) / TC_BK) * TC_BK;
-          if (weights_are_p) tma_load_2d(sp + sub * p_bytes, &map_p, &full_bar[kb], kx, p0);
-          else load_q(sp + k_sub * p_bytes + sub * q_bytes, &full_bar[kb], kx);
+          if (weights_are_p) tma_load_2d(sp + sub * p_bytes, &map_p, &full_bar[kb], k_of(kb, sub), p0);
+          else load_q(sp + k_sub * p_bytes + sub * q_bytes, &full_bar[kb], k_of(kb, sub));
         }
       }
+      __syncwarp();
     }
-    __syncwarp();
     pdl_wait();
-    if (lane < L) {
-      for (int kb = lane; kb < first_round; kb += L) {
+    for (int kb = 0; kb < first_round; ++kb) {
+      if (leader) {
         uint8_t* sp = smem + (size_t)kb * stage_bytes;
         for (int sub = 0; sub < k_sub; ++sub) {
-          const int kb64 = kb_begin + kb * k_sub + sub;
-          const int kx = (kb64 < kb_end ? kb64 : (prm.K + TC_BK - 1) / TC_BK) * TC_BK;
-          if (!weights_are_p) tma_load_2d(sp + sub * p_bytes, &map_p, &full_bar[kb], kx, p0);
-          else if (!ln) tma_load_2d(sp + k_sub * p_bytes + sub * q_bytes, &map_q, &full_bar[kb], kx, q0);
+          if (!weights_are_p) tma_load_2d(sp + sub * p_bytes, &map_p, &full_bar[kb], k_of(kb, sub), p0);
+          else if (!ln) tma_load_2d(sp + k_sub * p_bytes + sub * q_bytes, &map_q, &full_bar[kb], k_of(kb, sub), q0);
         }
       }
-      // later rounds: a stage is refilled when the MMAs have read it
-      for (int kb = first_round + lane; kb < num_kb; kb += L) {
-        const int s = kb % stages;
-        const uint32_t parity = ((kb / stages) & 1) ^ 1;
-        if (!mbar_wait(&empty_bar[s], parity, abort_flag)) break;
+      __syncwarp();
+    }
+    // later rounds: a stage is refilled when the MMAs have read it
+    int s = 0;
+    uint32_t parity = 0;
+    for (int kb = first_round; kb < num_kb; ++kb) {
+      if (!warp_mbar_wait(&empty_bar[s], parity, abort_flag, lane)) break;
+      if (leader) {
         uint8_t* sp = smem + (size_t)s * stage_bytes;
         mbar_expect_tx(&full_bar[s], stage_bytes);
         for (int sub = 0; sub < k_sub; ++sub) {
-          // a block past this split's end is asked for past the end of K: it arrives as zeros
-          const int kb64 = kb_begin + kb * k_sub + sub;
-          const int kx = (kb64 < kb_end ? kb64 : (prm.K + TC_BK - 1) / TC_BK) * TC_BK;
+          const int kx = k_of(kb, sub);
           tma_load_2d(sp + sub * p_bytes, &map_p, &full_bar[s], kx, p0);
           if (!ln) load_q(sp + k_sub * p_bytes + sub * q_bytes, &full_bar[s], kx);
         }
       }
+      __syncwarp();
+      if (++s == stages) {
+        s = 0;
+        parity ^= 1;
+      }
     }
-    __syncwarp();
     if (*abort_flag && lane == 0) {
       // give copies that are still in flight time to land before the block's shared memory goes away
       const long long t0 = clock64();
@@ -221,15 +225,13 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issuer: lane 0 waits and issues.  One thread runs a dependent
-    // instruction every few cycles, so the loop is kept to the bare minimum: the high half of the
-    // matrix descriptors is a constant, the low half is the stage's address plus a small offset.
+    // ---------------- MMA issuer: the warp walks, one lane issues
+    const bool leader = elect_one();
     const uint32_t idesc = umma_idesc(TC_BP, bq);
-    const uint32_t desc_hi = (uint32_t)(umma_desc(0) >> 32);
-    const uint32_t desc_lo0 = (uint32_t)umma_desc(smem_u32(smem));   // address field: bits 0..13, in 16-byte units
+    const uint32_t desc_lo0 = umma_desc_lo(smem_u32(smem));   // address field: bits 0..13, in 16-byte units
     const uint32_t stage_step = stage_bytes >> 4, p_step = p_bytes >> 4, q_step = q_bytes >> 4;
     const uint32_t q_off = (uint32_t)k_sub * p_step;
-    const uint32_t q_res0 = (uint32_t)umma_desc(smem_u32(q_region));
+    const uint32_t q_res0 = umma_desc_lo(smem_u32(q_region));
     int s = 0;
     uint32_t parity = 0, lo_stage = desc_lo0, accumulate = 0;
     bool ok = true;
@@ -237,22 +239,20 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
     for (int kb = 0; kb < num_kb && ok; ++kb) {
       if (!warp_mbar_wait(&full_bar[s], parity, abort_flag, lane)) break;
       tc_fence_after();
-      if (lane == 0) {
+      if (leader) {
         for (int sub = 0; sub < k_sub; ++sub) {
           const uint32_t pa = lo_stage + sub * p_step;
           const uint32_t qa = ln ? q_res0 + (uint32_t)(kb * k_sub + sub) * q_step : lo_stage + q_off + sub * q_step;
 #pragma unroll
-          for (int k = 0; k < TC_BK / 16; ++k) {
+          for (int k = 0; k < TC_BK / 16; ++k)
             // 16 bf16 = 32 bytes = 2 address units further along K inside the swizzled row
-            uint64_t da, db;
-            asm("mov.b64 %0, {%1, %2};" : "=l"(da) : "r"(pa + 2 * k), "r"(desc_hi));
-            asm("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(qa + 2 * k), "r"(desc_hi));
-            umma_bf16(tmem_base, da, db, idesc, accumulate);
-            accumulate = 1;
-          }
+            umma_bf16(tmem_base, umma_desc_of(pa + 2 * k), umma_desc_of(qa + 2 * k), idesc,
+                      k > 0 || sub > 0 ? 1u : accumulate);
         }
         umma_commit(&empty_bar[s]);  // frees the stage when these MMAs have read it
       }
+      __syncwarp();
+      accumulate = 1;
       lo_stage += stage_step;
       if (++s == stages) {
         s = 0;
@@ -260,9 +260,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
         lo_stage = desc_lo0;
       }
     }
-    if (lane == 0) {
-      umma_commit(&tmem_full_bar);  // arrives when every MMA above has finished
-    }
+    if (leader) umma_commit(&tmem_full_bar);  // arrives when every MMA above has finished
     __syncwarp();
   } else {
     // ---------------- epilogue warps: warp w owns TMEM lanes 32 * (w % 4) .. +32

@@ -112,8 +112,8 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   __shared__ int epi_ok_sh[4];
   __shared__ __align__(16) float bias_sh[256];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = cluster_rank();              // 0: the pair's first block (issues the MMAs), 1: the second
+  const int warp = warp_uniform((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int rank = warp_uniform(cluster_rank());   // 0: the pair's first block (issues the MMAs), 1: the second
   const int stages = prm.stages, bq = prm.bq, half = bq / 2;
   const uint32_t a_bytes = PR_BP * PR_BK * 2, w_bytes = (uint32_t)half * PR_BK * 2;
   const uint32_t stage_bytes = a_bytes + w_bytes;          // a multiple of 1024 (half % 8 == 0)
@@ -147,70 +147,83 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   cluster_arrive();
   cluster_wait();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_base_sh;
+  const uint32_t tmem_base = warp_uniform(tmem_base_sh);
   volatile int* abort_flag = &abort_sh;
   // Only the producer goes on before the kernel ahead has finished: it asks for the WEIGHT tiles of
   // the first stages (they do not depend on that kernel), and waits before it asks for activations.
   if (warp != 0) pdl_wait();
 
   if (warp == 0) {
-    // ---------------- TMA producer (one lane): this block's rows of the activations and its half of
-    // the weight tile; completion is counted at the first block's barrier, which expects both blocks' bytes
-    if (lane == 0) {
-      const int first_round = num_kb < stages ? num_kb : stages;
-      for (int kb = 0; kb < first_round; ++kb) {   // (the stages are all free)
+    // ---------------- TMA producer (the warp walks, one lane issues): this block's rows of the activations and its half
+    // of the weight tile; completion is counted at the first block's barrier, which expects both blocks' bytes
+    const bool leader = elect_one();
+    const uint32_t bar0 = warp_uniform(cluster_addr_of(&full_bar[0], 0));
+    const int first_round = num_kb < stages ? num_kb : stages;
+    for (int kb = 0; kb < first_round; ++kb) {   // (the stages are all free)
+      if (leader) {
         if (rank == 0) mbar_expect_tx(&full_bar[kb], 2 * stage_bytes);
-        tma_load_2d_pair(smem + (size_t)kb * stage_bytes + a_bytes, &map_w, cluster_addr_of(&full_bar[kb], 0),
-                         (kb_begin + kb) * PR_BK, qh0);
+        tma_load_2d_pair(smem + (size_t)kb * stage_bytes + a_bytes, &map_w, bar0 + kb * 8, (kb_begin + kb) * PR_BK, qh0);
       }
+      __syncwarp();
     }
-    __syncwarp();
     pdl_wait();
-    if (lane == 0) {
-      const int first_round = num_kb < stages ? num_kb : stages;
-      for (int kb = 0; kb < first_round; ++kb)
-        tma_load_2d_pair(smem + (size_t)kb * stage_bytes, &map_a, cluster_addr_of(&full_bar[kb], 0),
-                         (kb_begin + kb) * PR_BK, p0);
-      for (int kb = first_round; kb < num_kb; ++kb) {
-        const int s = kb % stages;
-        if (!mbar_wait(&empty_bar[s], ((kb / stages) & 1) ^ 1, abort_flag)) break;
+    for (int kb = 0; kb < first_round; ++kb) {
+      if (leader) tma_load_2d_pair(smem + (size_t)kb * stage_bytes, &map_a, bar0 + kb * 8, (kb_begin + kb) * PR_BK, p0);
+      __syncwarp();
+    }
+    int s = 0;
+    uint32_t parity = 0;
+    for (int kb = first_round; kb < num_kb; ++kb) {
+      if (!warp_mbar_wait(&empty_bar[s], parity, abort_flag, lane)) break;
+      if (leader) {
         uint8_t* sp = smem + (size_t)s * stage_bytes;
         if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * stage_bytes);
-        const uint32_t bar = cluster_addr_of(&full_bar[s], 0);
         const int kx = (kb_begin + kb) * PR_BK;
-        tma_load_2d_pair(sp, &map_a, bar, kx, p0);
-        tma_load_2d_pair(sp + a_bytes, &map_w, bar, kx, qh0);
+        tma_load_2d_pair(sp, &map_a, bar0 + s * 8, kx, p0);
+        tma_load_2d_pair(sp + a_bytes, &map_w, bar0 + s * 8, kx, qh0);
       }
-      if (*abort_flag) {
-        // give copies that are still in flight time to land before the block's shared memory goes away
-        const long long t0 = clock64();
-        while (clock64() - t0 < 2000000ll) {
-        }
+      __syncwarp();
+      if (++s == stages) {
+        s = 0;
+        parity ^= 1;
+      }
+    }
+    if (*abort_flag && lane == 0) {
+      // give copies that are still in flight time to land before the block's shared memory goes away
+      const long long t0 = clock64();
+      while (clock64() - t0 < 2000000ll) {
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issue, in the pair's first block only: M = 256 over the two blocks
-    if (rank == 0 && lane == 0) {
+    // ---------------- MMA issue, in the pair's first block only: M = 256 over the two blocks (the warp walks, one lane
+    // issues)
+    if (rank == 0) {
+      const bool leader = elect_one();
       const uint32_t idesc = umma_idesc(2 * PR_BP, bq);
-      uint32_t accumulate = 0;
-      bool ok = true;
-      for (int kb = 0; kb < num_kb && ok; ++kb) {
-        const int s = kb % stages;
-        if (!mbar_wait(&full_bar[s], (kb / stages) & 1, abort_flag)) {
-          ok = false;
-          break;
-        }
+      const uint32_t lo0 = umma_desc_lo(smem_u32(smem));
+      uint32_t lo = lo0, parity = 0, accumulate = 0;
+      int s = 0;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!warp_mbar_wait(&full_bar[s], parity, abort_flag, lane)) break;
         tc_fence_after();
-        const uint32_t pa = smem_u32(smem + (size_t)s * stage_bytes), wa = pa + a_bytes;
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < PR_BK / 16; ++k) {   // 16 bf16 = 32 bytes further along K inside the swizzled row
-          umma_bf16_pair(tmem_base, umma_desc(pa + k * 32), umma_desc(wa + k * 32), idesc, accumulate);
-          accumulate = 1;
+          for (int k = 0; k < PR_BK / 16; ++k)   // 16 bf16 = 32 bytes further along K inside the swizzled row
+            umma_bf16_pair(tmem_base, umma_desc_of(lo + 2 * k), umma_desc_of(lo + (a_bytes >> 4) + 2 * k), idesc,
+                           k > 0 ? 1u : accumulate);
+          umma_commit_pair(&empty_bar[s]);   // frees the stage, in both blocks, when these MMAs have read it
         }
-        umma_commit_pair(&empty_bar[s]);   // frees the stage, in both blocks, when these MMAs have read it
+        __syncwarp();
+        accumulate = 1;
+        lo += stage_bytes >> 4;
+        if (++s == stages) {
+          s = 0;
+          parity ^= 1;
+          lo = lo0;
+        }
       }
-      umma_commit_pair(&tmem_full_bar);     // arrives in both blocks when every MMA above has finished
+      if (leader) umma_commit_pair(&tmem_full_bar);     // arrives in both blocks when every MMA above has finished
     }
     __syncwarp();
   } else {
