@@ -28,7 +28,7 @@ namespace nib {
 
 constexpr int SK_WARPS = 8;
 constexpr int SK_MAX_ROWS = 128;
-constexpr int SK_LN_REG_WIDTH = 1024;   // rows up to this wide are normalised in registers ...
+constexpr int SK_LN_REG_WIDTH = 1024;   // rows up to this wide are normalised in registers (twice as wide for up to 8 rows) ...
 constexpr int SK_LN_MAX_WIDTH = 4096;   // ... wider ones, up to this, in shared memory
 constexpr int SK_MAX_SPLIT = 8;      // blocks of a cluster that split K
 
@@ -86,7 +86,8 @@ __host__ __device__ inline int skinny_ldx(int k_per) { return k_per + ((32 - k_p
 // rows' pieces are dealt the same way.
 // ROWS: the variant for steps of more than 16 rows, whose blocks each take a row block (the others keep
 // the code they had without it: a decode step of 8 rows is 0.7 % longer with the offset in every index).
-template <int NT, bool ROWS>
+// LN_NV: a lane's 16-byte pieces of a row that is normalised in registers (rows up to 128 * LN_NV wide).
+template <int NT, bool ROWS, int LN_NV>
 __global__ void __launch_bounds__(SK_WARPS * 32, 2)
 linear_skinny_kernel(const SkinnyParams prm) {
   pdl_trigger();
@@ -187,7 +188,7 @@ linear_skinny_kernel(const SkinnyParams prm) {
   // ---- the step's rows into shared memory as bfloat16 (normalised on the way if asked)
   for (int i = threadIdx.x; i < (NT * 8 - M) * (ldx / 8); i += blockDim.x)   // rows past the step: zeros
     reinterpret_cast<uint4*>(xs + (size_t)M * ldx)[i] = make_uint4(0, 0, 0, 0);
-  if (prm.ln_x != nullptr && prm.K > SK_LN_REG_WIDTH) {
+  if (prm.ln_x != nullptr && prm.K > 128 * LN_NV) {
     // Rows too wide for a lane's registers: a warp brings its row into a buffer of its own in shared
     // memory (summing on the way) and makes the other two passes there.
     __syncthreads();   // the norm's parameters are in place
@@ -224,11 +225,11 @@ linear_skinny_kernel(const SkinnyParams prm) {
     const int K = prm.K;
     for (int m = warp; m < M; m += SK_WARPS) {
       const float* src = prm.ln_x + (size_t)(prm.ln_rows ? prm.ln_rows[row0 + m] : row0 + m) * prm.ln_ldx;
-      // one read of the row into registers (K <= 1024: 32 floats a lane), then two passes on them
-      float v[32];
+      // one read of the row into registers, all of it asked for at once, then two passes on them
+      float v[4 * LN_NV];
       float sum = 0.0f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < LN_NV; ++j) {
         const int k = (j * 32 + lane) * 4;
         float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
         if (k < K) t = *reinterpret_cast<const float4*>(src + k);
@@ -238,7 +239,7 @@ linear_skinny_kernel(const SkinnyParams prm) {
       const float mean = prm.ln_beta != nullptr ? warp_sum(sum) / (float)K : 0.0f;   // (no shift: an RMS norm)
       float sq = 0.0f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < LN_NV; ++j) {
         const int k = (j * 32 + lane) * 4;
         if (k < K) {
 #pragma unroll
@@ -250,7 +251,7 @@ linear_skinny_kernel(const SkinnyParams prm) {
       }
       const float rstd = 1.0f / sqrtf(warp_sum(sq) / (float)K + prm.ln_eps);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < LN_NV; ++j) {
         const int k = (j * 32 + lane) * 4;
         if (k < K) {
           const float4 g = *reinterpret_cast<const float4*>(ln_gb + k);
@@ -438,12 +439,17 @@ linear_skinny_kernel(const SkinnyParams prm) {
 static int skinny_tiles(int M) { return M <= 8 ? 1 : 2; }
 static int skinny_row_blocks(int M) { const int r = skinny_tiles(M) * 8; return (M + r - 1) / r; }
 
+// Pieces a lane holds of a row that is normalised in registers.  Rows of 1,025 to 2,048 values: through a buffer per
+// warp in shared memory, a round trip for every few pieces and three walks, a block of GPT-2 XL's took about 1.5 us
+// longer; with 16 rows a block their 64 registers do not fit beside two tiles' sums.
+static int skinny_ln_nv(int NT, int K) { return NT == 1 && K > SK_LN_REG_WIDTH && K <= 2 * SK_LN_REG_WIDTH ? 16 : 8; }
+
 static size_t skinny_smem(int NT, int k_per, int K, bool ln, bool alias = false) {
   const size_t xs = (size_t)NT * 8 * skinny_ldx(k_per) * sizeof(bf16), red = (size_t)SK_WARPS * NT * 128 * sizeof(float);
   // (the other blocks' sums of a split K, kept without a split too: without them a decode step measured 1 % longer;
   // with the norm: its scale and shift, and for wide rows a buffer per warp)
   return (alias ? (xs > red ? xs : red) : xs + red) + (size_t)2 * NT * 128 * sizeof(float) +
-         (ln ? (size_t)(2 + (K > SK_LN_REG_WIDTH ? SK_WARPS : 0)) * K * sizeof(float) : 0);
+         (ln ? (size_t)(2 + (K > 128 * skinny_ln_nv(NT, K) ? SK_WARPS : 0)) * K * sizeof(float) : 0);
 }
 
 constexpr size_t SK_SMEM_LIMIT = 200 * 1024;
@@ -468,11 +474,11 @@ static int skinny_split(int M, int N, int K, bool ln) {
   return split;
 }
 
-template <int NT, bool ROWS>
+template <int NT, bool ROWS, int LN_NV = 8>
 static int launch_skinny(SkinnyParams prm, cudaStream_t stream) {
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(linear_skinny_kernel<NT, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(linear_skinny_kernel<NT, ROWS, LN_NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)SK_SMEM_LIMIT);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
@@ -509,7 +515,7 @@ static int launch_skinny(SkinnyParams prm, cudaStream_t stream) {
       q.dynamicSmemBytes = smem;
       q.attrs = attr + 1;      // the query takes the cluster shape only
       q.numAttrs = 1;
-      cudaError_t e = cudaOccupancyMaxActiveClusters(&n, linear_skinny_kernel<NT, ROWS>, &q);
+      cudaError_t e = cudaOccupancyMaxActiveClusters(&n, linear_skinny_kernel<NT, ROWS, LN_NV>, &q);
       if (e != cudaSuccess) { err = (int)e; return 0; }
       if (n < 1) { err = NIB_ERR_UNSUPPORTED_SIZE; return 0; }
       it = held.emplace(std::make_pair(cluster, smem), n).first;
@@ -539,7 +545,7 @@ static int launch_skinny(SkinnyParams prm, cudaStream_t stream) {
   const int walkers = n_tiles < cap ? n_tiles : cap;
   cfg.dynamicSmemBytes = smem;
   cfg.gridDim = dim3(walkers * prm.split, row_blocks);
-  cudaError_t e = cudaLaunchKernelEx(&cfg, linear_skinny_kernel<NT, ROWS>, prm);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, linear_skinny_kernel<NT, ROWS, LN_NV>, prm);
   if (e != cudaSuccess) return (int)e;
   NIB_LAUNCH_CHECK();
 }
@@ -596,7 +602,7 @@ extern "C" int nib_linear_skinny(int out_dtype, const void* a, int lda, const vo
   if (ln && ((ln_ldx & 3) || ((uintptr_t)ln_x & 15) || ((uintptr_t)ln_gamma & 15) || ((uintptr_t)ln_beta & 15)))
     return NIB_ERR_UNSUPPORTED_SIZE;
   switch (skinny_tiles(M)) {
-    case 1: return launch_skinny<1, false>(prm, stream);
+    case 1: return ln && skinny_ln_nv(1, K) == 16 ? launch_skinny<1, false, 16>(prm, stream) : launch_skinny<1, false>(prm, stream);
     default: return M > 16 ? launch_skinny<2, true>(prm, stream) : launch_skinny<2, false>(prm, stream);
   }
 }
