@@ -58,9 +58,9 @@ struct TcParams {
   int residual;
   int tma_store;     // 1: the epilogue stages the tile in shared memory and stores it with TMA
   int* status;
-  // Optional (swapped orientation only): output features from q_dim on are keys and values, which go
-  // straight to their slots in the paged cache instead of to `out` (the reference's QKV epilogue,
-  // crates/metal/src/shaders/batch.metal:155-164)
+  // Optional: output features from q_dim on are keys and values, which go straight to their slots in the paged cache
+  // instead of to `out` (the reference's QKV epilogue, crates/metal/src/shaders/batch.metal:155-164); in the plain
+  // orientation q_dim is a multiple of 64 and the head size of 16
   bf16* kv_cache;
   const int* kv_block_table;
   const int* kv_row_entry;
@@ -312,6 +312,16 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
       for (int c = (int)threadIdx.x - 64; c < bq; c += 128)
         bias_sh[c] = (prm.bias && first_split && q0 + c < prm.q_rows) ? prm.bias[q0 + c] : 0.0f;
     }
+    // the cache slot of this thread's row (two dependent look-ups in the step's tables), while the MMAs run
+    const bool kv_tile = !prm.swap && prm.kv_cache != nullptr && q0 + bq > prm.kv_q_dim;
+    long long kv_base = -1;   // element offset of (page, K, head 0, slot, 0) in the cache layer; -1: nothing is kept
+    if (kv_tile && p < prm.p_rows) {
+      const int pos = prm.kv_positions[p], entry = prm.kv_row_entry[p];   // (negative: a row of no request)
+      const int page = entry < 0 ? 0 : prm.kv_block_table[(size_t)entry * prm.kv_max_blocks + pos / prm.kv_page_size];
+      if (entry < 0) {}
+      else if (page < 0 || page >= prm.kv_n_pages) *prm.status = NIB_STATUS_BAD_PAGE;
+      else kv_base = (long long)kv_offset(page, 0, 0, pos % prm.kv_page_size, prm.kv_heads, prm.kv_page_size, prm.kv_head_dim);
+    }
     // the four epilogue warps go on only if all of them saw the accumulator complete
     if (lane == 0) epi_ok_sh[quarter] = mbar_wait(&tmem_full_bar, 0, abort_flag) ? 1 : 0;
     asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -349,7 +359,20 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
 #pragma unroll
               for (int j = 0; j < 16; ++j) v[j] = epilogue_act<ACT>(v[j]);
             }
-            if (prm.out_f32) {
+            if (kv_tile && q0 + c0 >= prm.kv_q_dim) {
+              // 16 consecutive values of one head of this row's key or value: 32 bytes into its cache slot
+              if (kv_base >= 0 && q0 + c0 < prm.q_rows) {
+                const int kv_dim = prm.kv_heads * prm.kv_head_dim, rem = q0 + c0 - prm.kv_q_dim;
+                const int which = rem / kv_dim, head = (rem % kv_dim) / prm.kv_head_dim, d = rem % prm.kv_head_dim;
+                bf16* dst = prm.kv_cache + kv_base +
+                            ((long long)which * prm.kv_heads + head) * prm.kv_page_size * prm.kv_head_dim + d;
+#pragma unroll
+                for (int j = 0; j < 16; j += 8)
+                  *reinterpret_cast<uint4*>(dst + j) =
+                      make_uint4(pack_bf16(v[j], v[j + 1]), pack_bf16(v[j + 2], v[j + 3]),
+                                 pack_bf16(v[j + 4], v[j + 5]), pack_bf16(v[j + 6], v[j + 7]));
+              }
+            } else if (prm.out_f32) {
               uint8_t* blk = smem + (size_t)(c0 / 32) * 16384 + (size_t)pl * 128;
 #pragma unroll
               for (int j = 0; j < 16; j += 4) {
@@ -372,7 +395,8 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
         asm volatile("bar.sync 1, 128;" ::: "memory");                // the four epilogue warps
         if (warp == 2 && lane == 0) {
           const int cols = prm.out_f32 ? 32 : 64;
-          for (int c = 0; c < bq && q0 + c < prm.q_rows; c += cols) {
+          const int n_out = prm.kv_cache != nullptr ? prm.kv_q_dim : prm.q_rows;   // columns that go to `out`
+          for (int c = 0; c < bq && q0 + c < n_out; c += cols) {
             const void* src = smem + (size_t)(c / cols) * 16384;
             if (prm.residual) tma_reduce_add_2d(&map_o, src, q0 + c, p0);
             else tma_store_2d(&map_o, src, q0 + c, p0);
@@ -575,8 +599,16 @@ static int launch_tc(int out_dtype, const void* a, int lda, const void* w, int l
   prm.kv_cache = nullptr;
   prm.kv_block_table = prm.kv_row_entry = prm.kv_positions = nullptr;
   prm.kv_max_blocks = prm.kv_q_dim = prm.kv_heads = prm.kv_head_dim = prm.kv_page_size = prm.kv_n_pages = 0;
+  const int esz = out_dtype == DT_F32 ? 4 : 2;
+  // TMA can store the tile if the output's rows are 16-byte multiples (it also clips a store at the
+  // tensor's edge in 16-byte pieces, so the row length must be a multiple too)
+  const bool tma_ok = ((uintptr_t)out & 15) == 0 && ((long)ldo * esz) % 16 == 0 && ((long)N * esz) % 16 == 0;
+  // keys and values from the plain orientation's epilogue: whole 16-value pieces of a head, queries in whole TMA stores
+  const bool kv_plain = kv != nullptr && M > 16 && ln == nullptr && fix == nullptr && tma_ok && N >= 64 && !(kv->q_dim & 63) &&
+                        !(kv->head_dim & 15) && !((uintptr_t)kv->cache & 15);
   if (kv != nullptr) {
-    if (M > 128 || out_dtype != DT_BF16 || act != ACT_NONE || residual) return NIB_ERR_BAD_ARGUMENT;
+    if (out_dtype != DT_BF16 || act != ACT_NONE || residual) return NIB_ERR_BAD_ARGUMENT;
+    if (M > 128 && !kv_plain) return NIB_ERR_UNSUPPORTED_SIZE;
     if (N != kv->q_dim + 2 * kv->heads * kv->head_dim) return NIB_ERR_BAD_ARGUMENT;
     prm.kv_cache = (bf16*)kv->cache;
     prm.kv_block_table = kv->block_table;
@@ -595,11 +627,7 @@ static int launch_tc(int out_dtype, const void* a, int lda, const void* w, int l
   // 128-feature tiles alone fill the device (the head); else activations on the M side even for 17 to 128
   // rows (one row tile, padded): the swapped product has N / 128 blocks, 38 for GPT-2 XL's q/k/v, the other
   // N / 64 and a split of K for the residual, and a step of an 80-token prompt takes 4.3 ms instead of 5.3.
-  prm.swap = seg_k == 0 && M <= 128 && (M <= 16 || kv != nullptr || ln != nullptr || fix != nullptr || (N + TC_BP - 1) / TC_BP >= 148);
-  const int esz = prm.out_f32 ? 4 : 2;
-  // TMA can store the tile if the output's rows are 16-byte multiples (it also clips a store at the
-  // tensor's edge in 16-byte pieces, so the row length must be a multiple too)
-  const bool tma_ok = ((uintptr_t)out & 15) == 0 && ((long)ldo * esz) % 16 == 0 && ((long)N * esz) % 16 == 0;
+  prm.swap = seg_k == 0 && M <= 128 && !kv_plain && (M <= 16 || kv != nullptr || ln != nullptr || fix != nullptr || (N + TC_BP - 1) / TC_BP >= 148);
   const int num_kb64 = (K + TC_BK - 1) / TC_BK;
   const void *p_base, *q_base;
   int p_ld, q_ld, splits = 1;
@@ -762,14 +790,15 @@ extern "C" int nib_linear_tc_segments(int out_dtype, const void* a, int lda, con
                    stream, seg_k);
 }
 
-// The general form for steps of at most 128 rows.  Any of three options may be on:
+// The general form for steps of at most 128 rows (with cache alone, any number of rows that the plain orientation
+// takes).  Any of three options may be on:
 //   * ln_x != null: the activations are LayerNorm(ln_x[ln_rows[m] or m]) (gamma, beta, eps), made in
 //     the kernel from the 32-bit residual stream (`a` is ignored);
 //   * cache != null: the fused query/key/value projection: the first q_dim features go to out, the
 //     rest to the rows' slots in one cache layer [n_pages, 2, n_kv_head, page_size, head_dim];
 //   * fix_partials != null: scratch (floats, and zeroed int counters that the kernel leaves zero)
 //     that lets K be split over blocks for outputs that are not a residual add.
-// Returns NIB_ERR_UNSUPPORTED_SIZE where the shape is not taken (more than 128 rows with ln_x, or
+// Returns NIB_ERR_UNSUPPORTED_SIZE where the shape is not taken (more than 128 rows with another option than cache, or
 // too much K for the resident activations); the caller then runs the plain kernels.
 extern "C" int nib_linear_tc_small(int out_dtype, const void* a, int lda, const void* w, int ldw, const float* bias,
                                    void* out, int ldo, int M, int N, int K, int act, int residual,
@@ -779,7 +808,8 @@ extern "C" int nib_linear_tc_small(int out_dtype, const void* a, int lda, const 
                                    int n_kv_head, int head_dim, int page_size, int n_pages, float* fix_partials,
                                    long long fix_floats, int* fix_counters, int fix_n_counters, int* status,
                                    cudaStream_t stream) {
-  if (M > 128) return NIB_ERR_UNSUPPORTED_SIZE;
+  if (M > 128 && (cache == nullptr || ln_x != nullptr || fix_partials != nullptr || out_dtype != DT_BF16 || act || residual))
+    return NIB_ERR_UNSUPPORTED_SIZE;
   LnSource ln{ln_x, ln_ldx, ln_gamma, ln_beta, ln_eps, ln_rows};
   KvTarget kv{cache, block_table, row_entry, positions, max_blocks, q_dim, n_kv_head, head_dim, page_size, n_pages};
   FixScratch fix{fix_partials, fix_floats, fix_counters, fix_n_counters};

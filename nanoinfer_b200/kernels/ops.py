@@ -567,8 +567,9 @@ def linear_skinny(a, norm, w, bias, out, M, act=ACT_NONE, residual=False, kv=Non
 def linear_small_tc(a, norm, w, bias, out, M, act=ACT_NONE, residual=False, kv=None, split=True) -> bool:
     """The tensor-core kernel for steps of at most 128 rows with its options: ``norm`` folds the
     LayerNorm before the product into the kernel, ``kv`` sends keys and values straight to the
-    cache, ``split`` lets K be split over blocks through scratch.  False if it does not apply."""
-    if M > SMALL_STEP_MAX_ROWS or not _small_inputs_ok(a, norm, w, out):
+    cache (alone, for any number of rows), ``split`` lets K be split over blocks through scratch.  False if it does
+    not apply."""
+    if (M > SMALL_STEP_MAX_ROWS and (kv is None or norm is not None or split)) or not _small_inputs_ok(a, norm, w, out):
         return False
     N, K = w.shape
     lib = library()
@@ -588,10 +589,6 @@ def linear_small_tc(a, norm, w, bias, out, M, act=ACT_NONE, residual=False, kv=N
     return True
 
 
-#: most rows for which the tcgen05 kernel writes keys and values from its epilogue (its swapped orientation)
-TC_KV_EPILOGUE_MAX_ROWS = 16
-
-
 def skinny_pays(M: int, N: int, K: int) -> bool:
     """Whether a product of at most 128 rows goes to the warp-level MMA kernel rather than to tcgen05.
     Measured in whole decode steps at widths 768, 1024 and 1600 (batch 16 to 64): up to 16 rows the MMA
@@ -599,7 +596,9 @@ def skinny_pays(M: int, N: int, K: int) -> bool:
     cluster: GPT-2 medium's second MLP product at 32 rows is 4 % of a step slower here, XL's 20 %) and the
     widest outputs (the head), where its 16-feature tiles read the rows too often; beyond 32 rows while a row
     block holds its rows unsplit.  Flipping one product's choice at a time at 24 to 128 rows and three widths
-    moves a step by less than 5 % where the other choice is better and by up to 97 % where it is worse."""
+    moves a step by less than 5 % where the other choice is better and by up to 97 % where it is worse.  (Alone, on
+    weights that the L2 holds, a norm and tcgen05 are ahead from 64 to 80 rows on, 10.6 against 12.5 us for 64 x 4096 x
+    1024; in a step, where the weights come from the memory, a prompt of 77 tokens takes 0.54 ms that way and 0.45 so.)"""
     if M <= 16:
         return True
     if N > 8192 or M > SKINNY_MAX_ROWS:
@@ -629,7 +628,7 @@ def _linear_small(a, norm, w, bias, out, M, act, residual, kv=None) -> bool:
             a, norm = norm.materialise(M), None
             if linear_skinny(a, None, w, bias, out, M, act, residual, kv):
                 return True
-    if M > TC_KV_EPILOGUE_MAX_ROWS or kv is None:
+    if kv is None or (M > 16 and (kv[4] % 64 or kv[0].shape[4] % 16)):
         return False          # the plain tensor-core call does as well
     if norm is not None:
         a, norm = norm.materialise(M), None
@@ -664,8 +663,7 @@ def linear_qkv(a: Optional[torch.Tensor], w: torch.Tensor, bias: Optional[torch.
                positions: torch.Tensor, status: torch.Tensor, norm: Optional[NormInput] = None) -> bool:
     """The fused q/k/v projection with the cache append in its epilogue: queries to out[:M, :q_dim],
     keys and values to their slots of ``cache``.  Returns False (and does nothing) where no fused
-    kernel applies: between 129 rows and the pair kernel's minimum (256), float32, or a shape the
-    tensor cores refuse."""
+    kernel applies: float32, or a shape the tensor cores refuse."""
     if cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
         return False
     kv = (cache, block_table, row_entry, positions, q_dim)

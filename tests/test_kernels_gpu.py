@@ -777,3 +777,37 @@ def test_fused_qkv_projection_for_many_rows(n_head, n_kv_head, hd, lens):
         want[page, 1, :, positions[t] % ps] = y[t, q_dim + kv_dim:].view(n_kv_head, hd)
     assert (cache.cpu().double() - want).abs().max() < 3e-2
     assert (out.cpu()[:, q_dim:] == 0).all()            # key and value columns of the buffer are not written
+
+
+@pytest.mark.parametrize("M", [17, 80, 128, 129, 255])
+@pytest.mark.parametrize("n_head, n_kv_head, hd, C", [(12, 12, 64, 768), (4, 2, 32, 72), (8, 1, 16, 1608)])
+def test_qkv_projection_of_17_to_255_rows_writes_the_cache_on_tcgen05(M, n_head, n_kv_head, hd, C):
+    """Rows on the MMA's M side: queries stored by TMA, keys and values from the epilogue into the rows' slots; every
+    seventh row is one of no request, which leaves nothing in the cache.  Rounding to bfloat16 (2^-9 of the value, and
+    sums of C products of 0.5 by 0.1 in 32 bits) bounds the difference."""
+    o = ops()
+    g = gen(M + hd)
+    ps, q_dim, kv_dim = 16, n_head * hd, n_kv_head * hd
+    N = q_dim + 2 * kv_dim
+    a = (torch.randn(M, C, generator=g) * 0.5).to(torch.bfloat16)
+    w = (torch.randn(N, C, generator=g) * 0.1).to(torch.bfloat16)
+    b = torch.randn(N, generator=g) * 0.1
+    pos0, n_blocks = 5, -(-(5 + M) // ps)
+    table = torch.randperm(n_blocks + 2, generator=g)[:n_blocks].to(torch.int32)[None]
+    entry = [-1 if t % 7 == 6 else 0 for t in range(M)]
+    cache = torch.zeros(n_blocks + 2, 2, n_kv_head, ps, hd, dtype=torch.bfloat16, device=DEV)
+    out = torch.zeros(M, N, dtype=torch.bfloat16, device=DEV)
+    kv = (cache, table.to(DEV), torch.tensor(entry, dtype=torch.int32, device=DEV),
+          torch.arange(pos0, pos0 + M, dtype=torch.int32, device=DEV), q_dim)
+    assert o.linear_small_tc(a.to(DEV), None, w.to(DEV), b.to(DEV), out, M, kv=kv, split=False)
+    assert int(o.status_word().item()) == 0
+    y = a.double() @ w.double().T + b.double()
+    tol = float(y.abs().max()) * 2.0 ** -8 + 1e-4
+    assert (out.cpu().double()[:, :q_dim] - y[:, :q_dim]).abs().max() < tol and (out.cpu()[:, q_dim:] == 0).all()
+    want = torch.zeros(cache.shape, dtype=torch.float64)
+    for t in range(M):
+        if entry[t] == 0:
+            at = int(table[0, (pos0 + t) // ps]), (pos0 + t) % ps
+            want[at[0], 0, :, at[1]] = y[t, q_dim:q_dim + kv_dim].view(n_kv_head, hd)
+            want[at[0], 1, :, at[1]] = y[t, q_dim + kv_dim:].view(n_kv_head, hd)
+    assert (cache.cpu().double() - want).abs().max() < tol
