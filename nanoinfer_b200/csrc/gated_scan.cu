@@ -12,6 +12,8 @@
 //
 // State per request (one row of the slot tensor): [taps - 1][channels] inputs of the convolution, oldest first,
 // then [head][V][NP] with NP = N rounded up to what the kernel variant holds (a multiple of 16).
+#include <type_traits>
+
 #include "api.h"
 #include "common.cuh"
 
@@ -196,43 +198,52 @@ gated_scan_kernel(const float* cv, int ldc, int q_off, int k_off, int v_off, int
     const float* base = sm + (size_t)(ck & 1) * SCAN_ROWS * ROW_F;
     const int rows = min(SCAN_ROWS, n - ck * SCAN_ROWS);
     float o[SCAN_ROWS], vj[SCAN_ROWS];
+    // (a chunk of eight rows has no branches between them, so that one row's read-out fills the waits of the next row's
+    // chain, and its vectors are there in time; every sum over N is four chains side by side)
+    auto walk = [&](auto full) {
+      constexpr bool FULL = decltype(full)::value;
 #pragma unroll
-    for (int rr = 0; rr < SCAN_ROWS; ++rr) {
-      o[rr] = 0.0f;
-      vj[rr] = 0.0f;
-      if (rr < rows) {
-        const float* kr = base + rr * ROW_F;
-        const float* qr = kr + NP;
-        const float a = kr[2 * NP + SCAN_COLS], wgt = kr[2 * NP + SCAN_COLS + 1];
-        vj[rr] = kr[2 * NP + jl];
-        float u;
-        if (DELTA) {
-          float ks = 0.0f;
+      for (int rr = 0; rr < SCAN_ROWS; ++rr) {
+        o[rr] = 0.0f;
+        vj[rr] = 0.0f;
+        if (FULL || rr < rows) {
+          const float* kr = base + rr * ROW_F;
+          const float* qr = kr + NP;
+          const float a = kr[2 * NP + SCAN_COLS], wgt = kr[2 * NP + SCAN_COLS + 1];
+          vj[rr] = kr[2 * NP + jl];
+          float4 k4[NPT / 4];
+#pragma unroll
+          for (int i = 0; i < NPT / 4; ++i) k4[i] = *reinterpret_cast<const float4*>(kr + 16 * i + 4 * p);
+          float u;
+          if (DELTA) {
+            float4 ks4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+            for (int i = 0; i < NPT / 4; ++i) {
+              ks4.x = fmaf(k4[i].x, S[4 * i], ks4.x);     ks4.y = fmaf(k4[i].y, S[4 * i + 1], ks4.y);
+              ks4.z = fmaf(k4[i].z, S[4 * i + 2], ks4.z); ks4.w = fmaf(k4[i].w, S[4 * i + 3], ks4.w);
+            }
+            float ks = (ks4.x + ks4.y) + (ks4.z + ks4.w);
+            ks += __shfl_xor_sync(0xffffffffu, ks, 1);
+            ks += __shfl_xor_sync(0xffffffffu, ks, 2);
+            u = wgt * (vj[rr] - a * ks);
+          } else {
+            u = wgt * vj[rr];
+          }
+          float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
           for (int i = 0; i < NPT / 4; ++i) {
-            const float4 k4 = *reinterpret_cast<const float4*>(kr + 16 * i + 4 * p);
-            ks = fmaf(k4.x, S[4 * i], ks); ks = fmaf(k4.y, S[4 * i + 1], ks);
-            ks = fmaf(k4.z, S[4 * i + 2], ks); ks = fmaf(k4.w, S[4 * i + 3], ks);
+            const float4 q4 = *reinterpret_cast<const float4*>(qr + 16 * i + 4 * p);
+            S[4 * i] = fmaf(a, S[4 * i], k4[i].x * u);         acc.x = fmaf(q4.x, S[4 * i], acc.x);
+            S[4 * i + 1] = fmaf(a, S[4 * i + 1], k4[i].y * u); acc.y = fmaf(q4.y, S[4 * i + 1], acc.y);
+            S[4 * i + 2] = fmaf(a, S[4 * i + 2], k4[i].z * u); acc.z = fmaf(q4.z, S[4 * i + 2], acc.z);
+            S[4 * i + 3] = fmaf(a, S[4 * i + 3], k4[i].w * u); acc.w = fmaf(q4.w, S[4 * i + 3], acc.w);
           }
-          ks += __shfl_xor_sync(0xffffffffu, ks, 1);
-          ks += __shfl_xor_sync(0xffffffffu, ks, 2);
-          u = wgt * (vj[rr] - a * ks);
-        } else {
-          u = wgt * vj[rr];
+          o[rr] = (acc.x + acc.y) + (acc.z + acc.w);
         }
-        float acc = 0.0f;
-#pragma unroll
-        for (int i = 0; i < NPT / 4; ++i) {
-          const float4 k4 = *reinterpret_cast<const float4*>(kr + 16 * i + 4 * p);
-          const float4 q4 = *reinterpret_cast<const float4*>(qr + 16 * i + 4 * p);
-          S[4 * i] = fmaf(a, S[4 * i], k4.x * u);         acc = fmaf(q4.x, S[4 * i], acc);
-          S[4 * i + 1] = fmaf(a, S[4 * i + 1], k4.y * u); acc = fmaf(q4.y, S[4 * i + 1], acc);
-          S[4 * i + 2] = fmaf(a, S[4 * i + 2], k4.z * u); acc = fmaf(q4.z, S[4 * i + 2], acc);
-          S[4 * i + 3] = fmaf(a, S[4 * i + 3], k4.w * u); acc = fmaf(q4.w, S[4 * i + 3], acc);
-        }
-        o[rr] = acc;
       }
-    }
+    };
+    if (rows == SCAN_ROWS) walk(std::true_type());
+    else walk(std::false_type());
     // the read-outs' sums over the four threads of a column, off the chain from row to row
 #pragma unroll
     for (int rr = 0; rr < SCAN_ROWS; ++rr) {
