@@ -528,7 +528,7 @@ SKINNY_MAX_ROWS = 128
 #: most rows of a step for which the dispatcher lets the few-row kernel normalise the rows itself (every
 #: row block of 16 its own rows: 24 launches fewer than with the norm as a kernel of its own)
 SKINNY_LN_MAX_ROWS = 128
-#: widest row that the few-row kernel normalises in a lane's registers
+#: widest row that the few-row kernel normalises in a lane's registers (up to 8 rows: twice that)
 SKINNY_LN_REGISTER_WIDTH = 1024
 PAIR_MIN_ROWS = 256      # the pair kernel's smallest step
 
