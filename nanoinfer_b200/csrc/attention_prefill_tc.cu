@@ -163,7 +163,6 @@ template <bool EX>
 __global__ void __launch_bounds__(AT_THREADS, 2)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                             const AtParams prm) {
-  pdl_trigger();
   extern __shared__ uint8_t at_smem_raw[];
   // tiles must start on a 1024-byte boundary for the 128-byte swizzle
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)at_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -214,6 +213,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   if (warp == 1) tmem_alloc(&tmem_base_sh, AT_TMEM_COLS);
   tc_fence_before();
   __syncthreads();
+  pdl_trigger();   // (behind the allocation: see tmem_alloc)
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(tmem_base_sh);
   if (warp != 0) pdl_wait();   // the queries, and this step's keys and values, come from the kernels ahead

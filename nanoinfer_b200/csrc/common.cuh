@@ -101,7 +101,8 @@ __device__ __forceinline__ size_t kv_offset(int page, int kv, int head, int slot
 }
 
 // Programmatic dependent launch.  Every kernel of the library starts with pdl_trigger() (the next
-// kernel in the stream may be scheduled and run its prologue while this one works) and calls
+// kernel in the stream may be scheduled and run its prologue while this one works; a kernel that takes
+// tensor memory calls it once it holds that, see tmem_alloc in tcgen05.cuh) and calls
 // pdl_wait() before its first access to global memory (which returns once the kernel before it has
 // finished and its writes are visible).  A step is a chain of a hundred short kernels, and this
 // hides each one's launch latency behind its predecessor.

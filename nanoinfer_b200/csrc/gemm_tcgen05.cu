@@ -102,7 +102,6 @@ template <int ACT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 linear_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
                  const __grid_constant__ CUtensorMap map_o, const TcParams prm) {
-  pdl_trigger();
   extern __shared__ uint8_t smem_raw[];
   // tiles must start on a 1024-byte boundary for the 128-byte swizzle
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -150,6 +149,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constan
   if (warp == 1) tmem_alloc(&tmem_base_sh, tmem_cols);
   tc_fence_before();
   __syncthreads();
+  pdl_trigger();   // (behind the allocation: see tmem_alloc)
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(tmem_base_sh);
   volatile int* abort_flag = &abort_sh;

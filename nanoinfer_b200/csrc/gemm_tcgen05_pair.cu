@@ -100,7 +100,6 @@ template <int ACT>
 __global__ void __launch_bounds__(PR_THREADS, 1)
 linear_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                       const __grid_constant__ CUtensorMap map_o, const PairParams prm) {
-  pdl_trigger();
   extern __shared__ uint8_t pr_smem_raw[];
   // tiles must start on a 1024-byte boundary for the 128-byte swizzle (the same offset in both blocks)
   uint8_t* smem = (uint8_t*)(((uintptr_t)pr_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -146,6 +145,7 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   // both blocks' barriers are initialised before either sends a load or a commit to the other
   cluster_arrive();
   cluster_wait();
+  pdl_trigger();   // (behind the allocation: see tmem_alloc)
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(tmem_base_sh);
   volatile int* abort_flag = &abort_sh;

@@ -51,6 +51,11 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
+// Waits, without a limit, until the columns are free.  So a block that holds columns must never wait for one that still
+// waits for some: the kernels behind are let go (pdl_trigger) only behind the __syncthreads() that follows the
+// allocation.  Their blocks start once every block of this kernel has let them go, and by then each holds its columns
+// and needs nothing but its own predecessors to finish and free them.  Let go before, a dependent that fits beside this
+// kernel's block on an SM could take the columns first and hold them while it waits for this kernel's end.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
                "r"(cols));
