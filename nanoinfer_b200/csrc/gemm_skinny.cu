@@ -225,6 +225,8 @@ linear_skinny_kernel(const SkinnyParams prm) {
     const int K = prm.K;
     for (int m = warp; m < M; m += SK_WARPS) {
       const float* src = prm.ln_x + (size_t)(prm.ln_rows ? prm.ln_rows[row0 + m] : row0 + m) * prm.ln_ldx;
+      // (rows that need more than eight pieces a lane are wider than eight: the first eight need no test)
+      auto inside = [&](int j, int k) { return (LN_NV > 8 && j < 8) || k < K; };
       // one read of the row into registers, all of it asked for at once, then two passes on them
       float v[4 * LN_NV];
       float sum = 0.0f;
@@ -232,7 +234,7 @@ linear_skinny_kernel(const SkinnyParams prm) {
       for (int j = 0; j < LN_NV; ++j) {
         const int k = (j * 32 + lane) * 4;
         float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (k < K) t = *reinterpret_cast<const float4*>(src + k);
+        if (inside(j, k)) t = *reinterpret_cast<const float4*>(src + k);
         v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
         sum += (t.x + t.y) + (t.z + t.w);
       }
@@ -241,7 +243,11 @@ linear_skinny_kernel(const SkinnyParams prm) {
 #pragma unroll
       for (int j = 0; j < LN_NV; ++j) {
         const int k = (j * 32 + lane) * 4;
-        if (k < K) {
+        if (LN_NV > 8) {   // (the order of the buffer above: a row's bits do not depend on how many there are)
+          const float mj = inside(j, k) ? mean : 0.0f;   // (zeros past the row: a branch a piece cost 0.3 us a launch)
+          const float d0 = v[4 * j] - mj, d1 = v[4 * j + 1] - mj, d2 = v[4 * j + 2] - mj, d3 = v[4 * j + 3] - mj;
+          sq += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
+        } else if (k < K) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float d = v[4 * j + e] - mean;
@@ -253,7 +259,7 @@ linear_skinny_kernel(const SkinnyParams prm) {
 #pragma unroll
       for (int j = 0; j < LN_NV; ++j) {
         const int k = (j * 32 + lane) * 4;
-        if (k < K) {
+        if (inside(j, k)) {
           const float4 g = *reinterpret_cast<const float4*>(ln_gb + k);
           const float4 b = *reinterpret_cast<const float4*>(ln_gb + K + k);
           __nv_bfloat162 lo = __floats2bfloat162_rn((v[4 * j] - mean) * rstd * g.x + b.x,

@@ -620,6 +620,33 @@ def test_few_row_product_in_row_blocks_gives_each_row_its_own_bits(M, N, K):
     assert int(o.status_word().item()) == 0
 
 
+@pytest.mark.parametrize("K", [1032, 1600, 2048])
+def test_wide_rows_are_normalised_to_the_same_bits_for_any_number_of_rows(K):
+    """Up to 8 rows a step of 1,025 to 2,048 values is normalised in registers, beyond that in shared memory.  The rows
+    are such that the order of the sum of squares shows: one value a lane whose square is 2^20, the others' squares a
+    third of its last bit, so that they vanish if they are added one by one.  The weights are the identity: the outputs
+    are the normalised rows themselves."""
+    o = ops()
+    from nanoinfer_b200.parts.base import Workspace
+    M = 64
+    x = 0.2 * (1 - 0.1 * torch.rand(M, K, generator=gen(K)))
+    x[:, 0:128:4] = 1024.0
+    w = torch.eye(K, dtype=torch.bfloat16, device=DEV)
+    gamma, bias = torch.ones(K, device=DEV), torch.zeros(K, device=DEV)
+    ws, xd = Workspace(torch.device(DEV)), x.to(DEV)
+
+    def product(rows):
+        out = torch.zeros(len(rows), K, dtype=torch.float32, device=DEV)
+        norm = o.NormInput(rows, gamma, None, 1e-5, ws, torch.bfloat16)     # (no shift: the squares stay as they are)
+        assert o.linear_skinny(None, norm, w, bias, out, len(rows))
+        return out
+
+    many = product(xd)
+    assert torch.equal(torch.cat([product(xd[i:i + 8].contiguous()) for i in range(0, M, 8)]), many)
+    assert torch.equal(product(xd[5:6].contiguous())[0], many[5])
+    assert int(o.status_word().item()) == 0
+
+
 SPLIT_SHAPES = [(1, 96, 768), (8, 768, 3072), (16, 768, 768), (20, 100, 1000), (33, 70, 3072), (64, 1000, 264),
                 (64, 768, 3072), (48, 2304, 768), (80, 768, 3072), (128, 100, 1000)]
 
