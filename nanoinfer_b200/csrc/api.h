@@ -324,8 +324,8 @@ int nib_scan_prepare(const float* proj, int ld, int a_off, int w_off, const floa
 int nib_gated_scan_padded(int N);
 int nib_gated_scan(int delta, const float* cv, int ldc, int q_off, int k_off, int v_off, int N, int V, int n_head,
                    int kq_ratio, const float* coef, const float* skip, float* state, long long state_stride,
-                   long long s_off, const int* entry_start, const int* entry_slot, int n_entries, float* out, int ldo,
-                   cudaStream_t stream);
+                   long long s_off, const int* entry_start, const int* entry_slot, int n_entries, int one_row,
+                   float* out, int ldo, cudaStream_t stream);
 int nib_gated_norm(int out_dtype, const float* o, int ldo, const float* gate, int ldg, const float* weight, int wlen,
                    int n_groups, int gs, float eps, int gate_first, float out_scale, void* out, int ld_out, int T,
                    cudaStream_t stream);

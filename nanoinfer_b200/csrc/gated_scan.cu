@@ -117,7 +117,7 @@ scan_prepare_kernel(const float* proj, int ld, int a_off, int w_off, const float
 }
 
 // ------------------------------------------------------------------ the recurrence
-constexpr int SCAN_ROWS = 8;      // rows staged at a time
+constexpr int SCAN_ROWS = 8;      // rows staged at a time (a step of one row an entry: one)
 constexpr int SCAN_COLS = 32;     // columns of S a block owns
 
 __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
@@ -128,8 +128,13 @@ __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) 
 // cv [T, ldc]: the rows' vectors: q (or C) of key/query head g at q_off + g N, k (or B) at k_off + g N, v (or x) of
 // head h at v_off + h V; head h reads key/query head h / kq_ratio.  coef [T, n_head, 2]: (a, w).  out [T, ldo]
 // float: o of head h at h V.  NPT: values of a column per thread (N <= 4 NPT).
-template <int NPT, bool DELTA>
-__global__ void __launch_bounds__(128)
+// ROWS: rows staged at a time: SCAN_ROWS, or one where every entry is one row.  A step of those is bound by the state's way
+// in and out, and the walk of whole chunks costs it registers that keep blocks away (delta rule, 64 requests, 12 heads of
+// 128 by 128: 20.5 us with it, 14.6 without; 18.4 when a chunk had a test a row).  At the largest size with the delta
+// rule the registers are held to three blocks an SM: with two (189 registers), eight portions of 100 rows were a second
+// wave (161 us instead of 109; one portion of 952 rows 614 instead of 626).
+template <int NPT, bool DELTA, int ROWS>
+__global__ void __launch_bounds__(128, NPT == 64 && DELTA ? 3 : 0)   // (0: the compiler's choice)
 gated_scan_kernel(const float* cv, int ldc, int q_off, int k_off, int v_off, int N, int V, int n_head, int kq_ratio,
                   const float* coef, const float* __restrict__ skip, float* state, long long state_stride,
                   long long s_off, const int* __restrict__ entry_start, const int* __restrict__ entry_slot,
@@ -145,7 +150,7 @@ gated_scan_kernel(const float* cv, int ldc, int q_off, int k_off, int v_off, int
   const int r0 = entry_start[e], n = entry_start[e + 1] - r0;
   const int g = h / kq_ratio;
   const int n_cols = min(SCAN_COLS, V - col0);
-  for (int i = tid; i < 2 * SCAN_ROWS * ROW_F; i += 128) sm[i] = 0.0f;   // (the tails behind N and V stay zero)
+  for (int i = tid; i < 2 * ROWS * ROW_F; i += 128) sm[i] = 0.0f;   // (the tails behind N and V stay zero)
   // the state belongs to this kernel alone: what it holds was written a step ago
   float S[NPT];
   float* sp = state + (size_t)entry_slot[e] * state_stride + s_off + ((size_t)h * V + (has_col ? j : 0)) * NP;
@@ -160,13 +165,13 @@ gated_scan_kernel(const float* cv, int ldc, int q_off, int k_off, int v_off, int
 
   // asks for the rows of chunk ck into buffer b
   auto stage = [&](int ck, int b) {
-    float* base = sm + (size_t)b * SCAN_ROWS * ROW_F;
-    const int rows = min(SCAN_ROWS, n - ck * SCAN_ROWS);
+    float* base = sm + (size_t)b * ROWS * ROW_F;
+    const int rows = min(ROWS, n - ck * ROWS);
     if (vec4) {
       const int nk = N >> 2, nv = n_cols >> 2, per = 2 * nk + nv;
       for (int i = tid; i < rows * per; i += 128) {
         const int rr = i / per, x = i % per;
-        const float* src = cv + (size_t)(r0 + ck * SCAN_ROWS + rr) * ldc;
+        const float* src = cv + (size_t)(r0 + ck * ROWS + rr) * ldc;
         float* dst = base + rr * ROW_F;
         if (x < nk) cp_async16(dst + 4 * x, src + k_off + g * N + 4 * x, true);
         else if (x < 2 * nk) cp_async16(dst + NP + 4 * (x - nk), src + q_off + g * N + 4 * (x - nk), true);
@@ -176,7 +181,7 @@ gated_scan_kernel(const float* cv, int ldc, int q_off, int k_off, int v_off, int
       const int per = 2 * N + n_cols;
       for (int i = tid; i < rows * per; i += 128) {
         const int rr = i / per, x = i % per;
-        const float* src = cv + (size_t)(r0 + ck * SCAN_ROWS + rr) * ldc;
+        const float* src = cv + (size_t)(r0 + ck * ROWS + rr) * ldc;
         float* dst = base + rr * ROW_F;
         if (x < N) cp_async4(dst + x, src + k_off + g * N + x);
         else if (x < 2 * N) cp_async4(dst + NP + (x - N), src + q_off + g * N + (x - N));
@@ -185,25 +190,25 @@ gated_scan_kernel(const float* cv, int ldc, int q_off, int k_off, int v_off, int
     }
     for (int i = tid; i < rows * 2; i += 128)
       cp_async4(base + (i >> 1) * ROW_F + 2 * NP + SCAN_COLS + (i & 1),
-                coef + ((size_t)(r0 + ck * SCAN_ROWS + (i >> 1)) * n_head + h) * 2 + (i & 1));
+                coef + ((size_t)(r0 + ck * ROWS + (i >> 1)) * n_head + h) * 2 + (i & 1));
     cp_async_commit();
   };
 
-  const int n_chunks = (n + SCAN_ROWS - 1) / SCAN_ROWS;
+  const int n_chunks = (n + ROWS - 1) / ROWS;
   if (n_chunks > 0) stage(0, 0);
   for (int ck = 0; ck < n_chunks; ++ck) {
     cp_async_wait<0>();
     __syncthreads();   // chunk ck has arrived, and every thread is done with the buffer that chunk ck + 1 goes to
     if (ck + 1 < n_chunks) stage(ck + 1, (ck + 1) & 1);
-    const float* base = sm + (size_t)(ck & 1) * SCAN_ROWS * ROW_F;
-    const int rows = min(SCAN_ROWS, n - ck * SCAN_ROWS);
-    float o[SCAN_ROWS], vj[SCAN_ROWS];
+    const float* base = sm + (size_t)(ck & 1) * ROWS * ROW_F;
+    const int rows = min(ROWS, n - ck * ROWS);
+    float o[ROWS], vj[ROWS];
     // (a chunk of eight rows has no branches between them, so that one row's read-out fills the waits of the next row's
     // chain, and its vectors are there in time; every sum over N is four chains side by side)
     auto walk = [&](auto full) {
       constexpr bool FULL = decltype(full)::value;
 #pragma unroll
-      for (int rr = 0; rr < SCAN_ROWS; ++rr) {
+      for (int rr = 0; rr < ROWS; ++rr) {
         o[rr] = 0.0f;
         vj[rr] = 0.0f;
         if (FULL || rr < rows) {
@@ -242,15 +247,15 @@ gated_scan_kernel(const float* cv, int ldc, int q_off, int k_off, int v_off, int
         }
       }
     };
-    if (rows == SCAN_ROWS) walk(std::true_type());
+    if (ROWS == 1 || rows == ROWS) walk(std::true_type());
     else walk(std::false_type());
     // the read-outs' sums over the four threads of a column, off the chain from row to row
 #pragma unroll
-    for (int rr = 0; rr < SCAN_ROWS; ++rr) {
+    for (int rr = 0; rr < ROWS; ++rr) {
       o[rr] += __shfl_xor_sync(0xffffffffu, o[rr], 1);
       o[rr] += __shfl_xor_sync(0xffffffffu, o[rr], 2);
       if (rr < rows && p == 0 && has_col)
-        out[(size_t)(r0 + ck * SCAN_ROWS + rr) * ldo + h * V + j] = o[rr] + d_skip * vj[rr];
+        out[(size_t)(r0 + ck * ROWS + rr) * ldo + h * V + j] = o[rr] + d_skip * vj[rr];
     }
   }
   if (has_col) {
@@ -343,39 +348,39 @@ extern "C" int nib_gated_scan_padded(int N) {
   return 0;
 }
 
-template <int NPT>
-static int launch_scan(int delta, dim3 grid, cudaStream_t stream, const float* cv, int ldc, int q_off, int k_off,
+template <int NPT, bool DELTA, int ROWS>
+static int launch_scan(dim3 grid, cudaStream_t stream, const float* cv, int ldc, int q_off, int k_off,
                        int v_off, int N, int V, int n_head, int kq_ratio, const float* coef, const float* skip,
                        float* state, long long state_stride, long long s_off, const int* entry_start,
                        const int* entry_slot, float* out, int ldo, int vec4) {
-  const size_t smem = (size_t)2 * SCAN_ROWS * (2 * 4 * NPT + SCAN_COLS + 4) * sizeof(float);
-  if (delta) {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(gated_scan_kernel<NPT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(gated_scan_kernel<NPT, true>, grid, dim3(128), smem, stream, cv, ldc, q_off, k_off, v_off, N, V, n_head,
-               kq_ratio, coef, skip, state, state_stride, s_off, entry_start, entry_slot, out, ldo, vec4);
-  } else {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(gated_scan_kernel<NPT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(gated_scan_kernel<NPT, false>, grid, dim3(128), smem, stream, cv, ldc, q_off, k_off, v_off, N, V, n_head,
-               kq_ratio, coef, skip, state, state_stride, s_off, entry_start, entry_slot, out, ldo, vec4);
-  }
+  const size_t smem = (size_t)2 * ROWS * (2 * 4 * NPT + SCAN_COLS + 4) * sizeof(float);
+  auto kernel = gated_scan_kernel<NPT, DELTA, ROWS>;
+  if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  launch_pdl(kernel, grid, dim3(128), smem, stream, cv, ldc, q_off, k_off, v_off, N, V, n_head, kq_ratio, coef, skip, state,
+             state_stride, s_off, entry_start, entry_slot, out, ldo, vec4);
   NIB_LAUNCH_CHECK();
 }
 
-// s_off: floats from the start of a slot's row to the matrices [n_head][V][nib_gated_scan_padded(N)].
+// s_off: floats from the start of a slot's row to the matrices [n_head][V][nib_gated_scan_padded(N)].  one_row: every
+// entry is one row.
 extern "C" int nib_gated_scan(int delta, const float* cv, int ldc, int q_off, int k_off, int v_off, int N, int V,
                               int n_head, int kq_ratio, const float* coef, const float* skip, float* state,
                               long long state_stride, long long s_off, const int* entry_start, const int* entry_slot,
-                              int n_entries, float* out, int ldo, cudaStream_t stream) {
+                              int n_entries, int one_row, float* out, int ldo, cudaStream_t stream) {
   if (n_entries <= 0) return 0;
   const int NP = nib_gated_scan_padded(N);
   if (NP == 0 || N <= 0 || V <= 0 || n_head > 65535 || n_entries > 65535) return NIB_ERR_UNSUPPORTED_SIZE;
   if (kq_ratio <= 0 || n_head % kq_ratio != 0 || (s_off & 3) || (state_stride & 3)) return NIB_ERR_BAD_ARGUMENT;
   const int vec4 = !((N | V | ldc | q_off | k_off | v_off) & 3) && (((uintptr_t)cv & 15) == 0);
   const dim3 grid((V + SCAN_COLS - 1) / SCAN_COLS, n_head, n_entries);
-#define NIB_SCAN(NPT) return launch_scan<NPT>(delta, grid, stream, cv, ldc, q_off, k_off, v_off, N, V, n_head, kq_ratio, \
-                                              coef, skip, state, state_stride, s_off, entry_start, entry_slot, out, ldo, vec4)
+#define NIB_SCAN_AS(NPT, DELTA, ROWS)                                                                                  \
+  return launch_scan<NPT, DELTA, ROWS>(grid, stream, cv, ldc, q_off, k_off, v_off, N, V, n_head, kq_ratio, coef, skip, \
+                                       state, state_stride, s_off, entry_start, entry_slot, out, ldo, vec4)
+#define NIB_SCAN(NPT)                                     \
+  if (delta && one_row) NIB_SCAN_AS(NPT, true, 1);        \
+  if (delta) NIB_SCAN_AS(NPT, true, SCAN_ROWS);           \
+  if (one_row) NIB_SCAN_AS(NPT, false, 1);                \
+  NIB_SCAN_AS(NPT, false, SCAN_ROWS)
   switch (NP) {
     case 16: NIB_SCAN(4);
     case 32: NIB_SCAN(8);
@@ -387,6 +392,7 @@ extern "C" int nib_gated_scan(int delta, const float* cv, int ldc, int q_off, in
     default: NIB_SCAN(64);
   }
 #undef NIB_SCAN
+#undef NIB_SCAN_AS
 }
 
 extern "C" int nib_gated_norm(int out_dtype, const float* o, int ldo, const float* gate, int ldg, const float* weight,

@@ -128,7 +128,7 @@ _SIGNATURES = {
                          _c_int, _c_int, _c_ptr, _c_int, _c_ptr],
     "nib_gated_scan_padded": [_c_int],
     "nib_gated_scan": [_c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr,
-                       _c_ptr, ctypes.c_longlong, ctypes.c_longlong, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr],
+                       _c_ptr, ctypes.c_longlong, ctypes.c_longlong, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_ptr],
     "nib_gated_norm": [_c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_float, _c_int, _c_float,
                        _c_ptr, _c_int, _c_int, _c_ptr],
     "nib_moe_down": [_c_int, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_ptr],
@@ -1827,7 +1827,8 @@ def gated_scan(delta: bool, cv: torch.Tensor, q_off: int, k_off: int, v_off: int
     _check(library().nib_gated_scan(int(bool(delta)), _ptr(cv), cv.stride(0), int(q_off), int(k_off), int(v_off), int(n),
                                     int(v), int(n_head), int(kq_ratio), _ptr(coef), _ptr(skip), _ptr(state),
                                     state.stride(0), int(s_off), _ptr(ctx.entry_start), _ptr(ctx.entry_slot),
-                                    ctx.n_entries, _ptr(out), out.stride(0), _stream()), "gated_scan")
+                                    ctx.n_entries, int(ctx.n_rows == ctx.n_entries), _ptr(out), out.stride(0), _stream()),
+           "gated_scan")   # (every entry has a row, so as many rows as entries means one each)
 
 
 def gated_norm(o: torch.Tensor, gate: Optional[torch.Tensor], weight: torch.Tensor, n_groups: int, group_size: int,

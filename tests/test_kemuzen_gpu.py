@@ -154,6 +154,30 @@ def _scan_reference(delta, q, k, v, a, w, skip, kq_ratio):
 
 
 @pytest.mark.parametrize("delta", [True, False])
+@pytest.mark.parametrize("N", [64, 100, 256])
+@pytest.mark.parametrize("rows", [1, 7])
+def test_recurrence_gives_an_entry_the_same_bits_beside_a_longer_one(rows, N, delta):
+    """Steps in which no entry can have a whole chunk of eight rows run on code of their own; beside an entry of eight
+    or nine rows the same entry runs on the other."""
+    from nanoinfer_b200.kernels import ops
+
+    torch.manual_seed(N + rows)
+    H, V, NP = 2, 40, ops.gated_scan_padded(N)
+    cv = torch.randn(rows + 9, 2 * H * N + H * V, device=DEV) * N ** -0.5
+    coef = torch.rand(rows + 9, H, 2, device=DEV)
+    begin = torch.randn(2, H * V * NP, device=DEV) * 0.1
+    got = []
+    for lens in ([rows], [rows, 8], [rows, 9]):
+        state, T = begin.clone(), sum(lens)
+        ctx = step_ctx(lens, [0] * T, slots=list(range(len(lens))))
+        out = torch.zeros(T, H * V, device=DEV)
+        ops.gated_scan(delta, cv[:T].contiguous(), 0, H * N, 2 * H * N, N, V, H, 1, coef[:T].contiguous(), None, state, 0, ctx, out)
+        got.append((out[:rows], state[0]))
+    for out, state in got[1:]:
+        assert torch.equal(out, got[0][0]) and torch.equal(state, got[0][1])
+
+
+@pytest.mark.parametrize("delta", [True, False])
 @pytest.mark.parametrize("H,G,N,V", [(2, 2, 16, 24), (4, 2, 20, 10), (1, 1, 64, 64), (3, 1, 50, 33), (2, 1, 256, 16),
                                      (6, 3, 48, 48), (2, 2, 128, 70)])
 def test_recurrence_kernel_carries_its_matrices_in_the_slot(H, G, N, V, delta):
