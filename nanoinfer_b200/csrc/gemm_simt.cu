@@ -15,6 +15,8 @@
 //   rows x N x K:  4 x 768 x 768: 13.7, 3.2     4 x 2304 x 768: 13.7, 4.0    4 x 768 x 3072: 52.6, 7.0
 //   4 x 50257 x 768: 57, 34     8 x 50257 x 768: 57, 49     212 x 2304 x 768: 111, 41    212 x 768 x 3072: 229, 54
 //   600 x 3072 x 768: 223, 103    2400 x 3072 x 768: 471, 333 (34 TFLOP/s)
+#include <atomic>
+
 #include "api.h"
 #include "common.cuh"
 
@@ -336,16 +338,26 @@ static int launch_rows(const InT* a, int lda, const InT* w, int ldw, const float
   if (allowed != cudaSuccess) return (int)allowed;
   const int n_st = (K + RW_K - 1) / RW_K, a_stages = n_st < 2 ? 1 : 2, groups = (N + RW_F - 1) / RW_F;
   // One group of features a block while the device holds them all at once (a block that has one round needs one stage
-  // of weights); else as many blocks as it holds, with two stages.
+  // of weights); else as many blocks as it holds, with two stages.  What an SM holds is asked for once for each size of a
+  // stage (registers count too: with 8 and 16 rows they leave room for two blocks).
+  cudaError_t err = cudaSuccess;
   auto held = [&](int w_stages) {
-    const size_t n = (size_t)(227 * 1024) / (rows_smem<ROWS>(w_stages, a_stages, K) + 1024);
-    return 148 * (int)(n < 1 ? 1 : n > 8 ? 8 : n);
+    static std::atomic<int> kept[5][2];      // [eighths of a stage that K fills, less one; several stages][stages of weights]
+    std::atomic<int>& slot = kept[n_st > 1 ? 4 : rows_pitch(K) / (8 * SEG_LD) - 1][w_stages - 1];
+    int n = slot.load(std::memory_order_relaxed);
+    if (n == 0) {
+      err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 256, rows_smem<ROWS>(w_stages, a_stages, K));
+      if (err != cudaSuccess) return 148;
+      slot.store(n = n < 1 ? 1 : n, std::memory_order_relaxed);
+    }
+    return 148 * n;
   };
   int w_stages = n_st > 1 ? 2 : 1, blocks = groups;
   if (groups > held(w_stages)) {
     w_stages = 2;
     blocks = held(2);
   }
+  if (err != cudaSuccess) return (int)err;
   launch_pdl(kernel, dim3(blocks), dim3(256), rows_smem<ROWS>(w_stages, a_stages, K), stream, a, lda, w, ldw, bias, out, ldo, M,
              N, K, act, residual, w_stages);
   NIB_LAUNCH_CHECK();

@@ -128,7 +128,8 @@ def test_linear_rows_do_not_depend_on_the_batch():
                 assert torch.equal(few, full[m0:m0 + n]), (act, residual, m0, n)
 
 
-@pytest.mark.parametrize("N, K", [(1, 1), (9, 31), (65, 33), (130, 260), (72, 1024), (2400, 96), (40, 1100), (24, 3076), (9600, 40)])
+@pytest.mark.parametrize("N, K", [(1, 1), (9, 31), (65, 33), (130, 260), (72, 1024), (2400, 96), (40, 1100), (24, 3076), (9600, 40),
+                                  (2376, 768), (4800, 1600), (4808, 2100)])
 @pytest.mark.parametrize("pad", [0, 1])
 def test_linear_in_32_bits_at_the_edges_of_segments_stages_and_tiles(N, K, pad):
     """Rows around every change of kernel and tile, K around a segment (32) and a stage (1,024) of it, outputs narrow
