@@ -6,7 +6,7 @@
 // the layout the reference transposes to at load (crates/core/src/weights.rs:1-9),
 // and the product is the reference's x . W^T + b (crates/core/src/kernels/reference.rs:26-37).
 //
-// The order of an output's sum depends on K alone, never on the other rows of the batch, and is the same in both
+// The order of an output's sum depends on K alone, never on the other rows of the batch, and is the same in the three
 // kernels below: K is cut into segments of 32, each one chain of fused multiply-adds in index order from zero; the
 // segments of a quarter of K (whole segments, rounded up) are added in order, and the four quarters are.  Chains of
 // 32 instead of one of K make room for many threads an output, and the sum more exact (N(0, 1) values, against 64
@@ -16,6 +16,7 @@
 //   4 x 50257 x 768: 57, 34     8 x 50257 x 768: 57, 49     212 x 2304 x 768: 111, 41    212 x 768 x 3072: 229, 54
 //   600 x 3072 x 768: 223, 103    2400 x 3072 x 768: 471, 333 (34 TFLOP/s)
 #include <atomic>
+#include <type_traits>
 
 #include "api.h"
 #include "common.cuh"
@@ -325,6 +326,109 @@ linear_simt_rows_kernel(const InT* a, int lda, const InT* __restrict__ w, int ld
   }
 }
 
+// ---------------------------------------------------------------------- at most 16 rows and few chunks of K
+// With K of one or two hundred a block of the kernel above has segments for a few of its threads only, and a wide output
+// many blocks.  Here a block owns 64 features and every thread one feature for ROWS / 4 of the step's rows; K comes in
+// chunks of 64 that are asked for two chunks ahead (registers).  A chunk costs about 1.05 us whatever the rows (1.35 with
+// 16 rows) while a block has an SM to itself: a chain of round trips, and bound by it.
+constexpr int FB_N = 64, FB_K = 2 * SEG;
+
+template <typename InT, typename OutT, int ROWS>
+__global__ void __launch_bounds__(256)
+linear_simt_features_kernel(const InT* a, int lda, const InT* __restrict__ w, int ldw,
+                            const float* __restrict__ bias, OutT* out, int ldo, int M, int N, int K,
+                            int act, int residual) {
+  constexpr int RPT = ROWS / 4;                      // rows per thread
+  constexpr int WPT = FB_N * FB_K / 256;             // weight values a thread stages per chunk: 16
+  constexpr int APT = (ROWS * FB_K + 255) / 256;     // values of the step's rows per thread and chunk
+  pdl_trigger();
+  __shared__ float Ws[2][FB_N][FB_K + 1];
+  __shared__ __align__(16) float As[2][ROWS][FB_K];
+  const int tid = threadIdx.x, n0 = blockIdx.x * FB_N;
+  const int f = tid % FB_N, rg = tid / FB_N;
+  const int lk = tid % FB_K, lr = tid / FB_K;        // staging: column of the chunk, first of the rows (step 4)
+  const int per_quarter = quarter_segments(K);
+  int left = per_quarter;                            // segments until the quarter ends
+  float wreg[2][WPT], areg[2][APT];
+  // asks for chunk c (columns c * 64 ...) into the register set `s`: weights do not depend on the kernel
+  // ahead, the step's rows do
+  auto ask_w = [&](int c, int s) {
+#pragma unroll
+    for (int j = 0; j < WPT; ++j) {
+      const int n = n0 + lr + 4 * j, k = c * FB_K + lk;
+      wreg[s][j] = (n < N && k < K) ? to_float(w[(size_t)n * ldw + k]) : 0.0f;
+    }
+  };
+  auto ask_a = [&](int c, int s) {
+#pragma unroll
+    for (int j = 0; j < APT; ++j) {
+      const int m = lr + 4 * j, k = c * FB_K + lk;
+      areg[s][j] = (m < M && m < ROWS && k < K) ? to_float(a[(size_t)m * lda + k]) : 0.0f;
+    }
+  };
+  const int n_chunks = (K + FB_K - 1) / FB_K;
+  ask_w(0, 0);
+  if (n_chunks > 1) ask_w(1, 1);
+  pdl_wait();
+  ask_a(0, 0);
+  if (n_chunks > 1) ask_a(1, 1);
+  float total[RPT], quarter[RPT];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) total[i] = quarter[i] = 0.0f;
+  // one chunk: the registers of set S go to buffer S, the chunk after next is asked for into them, and
+  // the chunk's two segments are added (S is a constant of the code, so that the sets stay in registers)
+  auto chunk = [&](int c, auto S) {
+    constexpr int s = decltype(S)::value;
+#pragma unroll
+    for (int j = 0; j < WPT; ++j) Ws[s][lr + 4 * j][lk] = wreg[s][j];
+#pragma unroll
+    for (int j = 0; j < APT; ++j) As[s][lr + 4 * j][lk] = areg[s][j];
+    if (c + 2 < n_chunks) {
+      ask_w(c + 2, s);
+      ask_a(c + 2, s);
+    }
+    __syncthreads();          // (two buffers by turns: a buffer is written again two chunks later, a barrier between)
+    float acc[2][RPT];        // the chunk's two segments (past the end of K: zeros, which change nothing)
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) acc[0][i] = acc[1][i] = 0.0f;
+#pragma unroll 2
+    for (int k = 0; k < SEG; k += 4) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float* ws = &Ws[s][f][h * SEG + k];
+        const float4 wv = make_float4(ws[0], ws[1], ws[2], ws[3]);
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+          acc[h][i] = fma4(*reinterpret_cast<const float4*>(&As[s][rg * RPT + i][h * SEG + k]), wv, acc[h][i]);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) quarter[i] += acc[h][i];
+      if (--left == 0) {
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          total[i] += quarter[i];
+          quarter[i] = 0.0f;
+        }
+        left = per_quarter;
+      }
+    }
+  };
+  for (int c = 0; c < n_chunks; c += 2) {
+    chunk(c, std::integral_constant<int, 0>());
+    if (c + 1 < n_chunks) chunk(c + 1, std::integral_constant<int, 1>());
+  }
+  const int n = n0 + f;
+  if (n >= N) return;
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int m = rg * RPT + i;
+    if (m < M) finish(total[i] + quarter[i], bias, out, ldo, m, n, act, residual);
+  }
+}
+
 template <typename K>
 static cudaError_t allow_smem(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -363,6 +467,32 @@ static int launch_rows(const InT* a, int lda, const InT* w, int ldw, const float
   NIB_LAUNCH_CHECK();
 }
 
+template <typename InT, typename OutT, int ROWS, bool VEC>
+static int launch_features(const InT* a, int lda, const InT* w, int ldw, const float* bias, OutT* out, int ldo, int M, int N,
+                           int K, int act, int residual, cudaStream_t stream) {
+  launch_pdl(linear_simt_features_kernel<InT, OutT, ROWS>, dim3((N + FB_N - 1) / FB_N), dim3(256), 0, stream, a, lda, w, ldw,
+             bias, out, ldo, M, N, K, act, residual);
+  NIB_LAUNCH_CHECK();
+}
+
+// Up to how many chunks of K (64) the kernel above is ahead.  It costs about a chunk's round trip a chunk; the other one
+// about the same whatever K up to several hundred, but a group of eight features at a time, so that it falls behind where
+// outputs are wide or rows many; without asynchronous copies (16-bit values, odd pitches) sooner.  us, this one and the
+// other: N = 768, K = 64: 1 row 1.80, 1.91, 16 rows 2.45, 3.00; K = 128, 16 rows 3.46, 3.11.  N = 3,072: K = 128, 4 rows 2.86,
+// 3.35, 16 rows 3.52, 5.58; K = 256, 16 rows 6.31, 6.05.  N = 9,600: K = 64, 8 rows 3.05, 6.76; K = 128, 1 row 4.29, 3.86, 4 rows
+// 4.39, 5.01; K = 256, 8 rows 9.32, 7.57, 16 rows 9.87, 12.34; K = 384, 16 rows 14.4, 13.6.  N = 50,257, K = 768, 16 rows 83, 86.
+// bfloat16: N = 768, K = 33: 8 rows 2.12, 3.67; K = 100: 4 rows 2.96, 2.41, 8 rows 3.00, 3.60; N = 9,600, K = 130: 8 rows 7.24, 10.07.
+template <typename InT, bool VEC>
+static bool features_pay(int M, int N, int K) {
+  const bool wide = N >= 8192, middle = N >= 2048, half = sizeof(InT) == 2;
+  int most;
+  if (M <= 2) most = half && wide ? 2 : 1;
+  else if (M <= 4) most = wide || (middle && (VEC || half)) ? 2 : 1;
+  else if (M <= 8) most = half ? (wide ? 3 : 2) : VEC ? (wide ? 3 : middle ? 2 : 1) : wide ? 2 : 1;
+  else most = VEC && N >= 32768 ? 12 : wide ? 5 : middle ? 3 : VEC ? 1 : 2;
+  return (K + FB_K - 1) / FB_K <= most;
+}
+
 template <typename InT, typename OutT, int TM, bool VEC>
 static int launch_tile(const InT* a, int lda, const InT* w, int ldw, const float* bias, OutT* out, int ldo, int M, int N,
                        int K, int act, int residual, cudaStream_t stream) {
@@ -382,6 +512,7 @@ template <typename InT, typename OutT, bool VEC>
 static int launch_any(const InT* a, int lda, const InT* w, int ldw, const float* bias, OutT* out, int ldo, int M, int N,
                       int K, int act, int residual, cudaStream_t stream) {
 #define NIB_SIMT(F, P) F<InT, OutT, P, VEC>(a, lda, w, ldw, bias, out, ldo, M, N, K, act, residual, stream)
+  if (M <= 16 && features_pay<InT, VEC>(M, N, K)) return M <= 8 ? NIB_SIMT(launch_features, 8) : NIB_SIMT(launch_features, 16);
   if (M <= 2) return NIB_SIMT(launch_rows, 2);
   if (M <= 4) return NIB_SIMT(launch_rows, 4);
   if (M <= 8) return NIB_SIMT(launch_rows, 8);

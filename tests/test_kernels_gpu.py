@@ -153,6 +153,30 @@ def test_linear_in_32_bits_at_the_edges_of_segments_stages_and_tiles(N, K, pad):
         last = out[:M].clone()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N, K", [(1, 1), (63, 33), (65, 64), (129, 100), (2050, 128), (2048, 190), (8200, 65), (8192, 320)])
+@pytest.mark.parametrize("pad", [0, 1])
+def test_linear_of_few_rows_and_few_chunks_of_k(N, K, pad, dtype):
+    """A feature a thread, K in chunks of 64: the bits of the kernel that takes the same rows in a larger step (32-bit
+    outputs of both value types), up to and beyond the chunks from which on that one takes them itself."""
+    g = gen(6)
+    o = ops()
+    w = torch.randn(N, K + pad, generator=g).to(dtype)[:, :K].to(DEV)
+    a = torch.randn(17, K + pad, generator=g).to(dtype)[:, :K].to(DEV)
+    bias = torch.randn(N, generator=g).to(DEV)
+    base = torch.randn(17, N, generator=g).to(DEV)
+    many = base.clone()
+    o.linear_simt(a, w, bias, many, 17, o.ACT_GELU_TANH, True)
+    a64, w64 = a.double(), w.double()
+    sums = torch.zeros(17, N, device=DEV)
+    o.linear_simt(a, w, None, sums, 17)
+    assert bool(((sums.double() - a64 @ w64.T).abs() <= 48 * 2.0 ** -24 * (a64.abs() @ w64.abs().T) + 1e-30).all())
+    for M in (1, 2, 3, 4, 5, 8, 9, 16):
+        few = base.clone()
+        o.linear_simt(a[:M], w, bias, few, M, o.ACT_GELU_TANH, True)
+        assert torch.equal(few[:M], many[:M]) and torch.equal(few[M:], base[M:]), M
+
+
 def paged_case(dtype, n_head, n_kv_head, hd, page_size, lengths, q_lens, seed):
     """Requests of the given lengths whose last q_lens tokens are this step's rows; pages are dealt
     out in a shuffled order so that a request's blocks lie scattered."""
