@@ -31,6 +31,7 @@ struct PairParams {
   int bq;            // columns of the tile = MMA N (a multiple of 32, at most 256); a block loads bq / 2 weight rows
   int stages;
   int kb_per_split;  // 64-wide K blocks per split of K (grid.z splits; their tiles are summed by reduce-add)
+  int kb_first;      // how many of them go to the first accumulator; the others to a second one beside it
   int out_f32;
   const float* bias;
   int residual;
@@ -123,8 +124,9 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const int kb_end = min((prm.K + PR_BK - 1) / PR_BK, kb_begin + prm.kb_per_split);
   const int num_kb = kb_end - kb_begin;
   const bool first_split = blockIdx.z == 0;
+  const bool second = num_kb > prm.kb_first;     // (the last split of K may be too short for one)
   uint32_t tmem_cols = 32;
-  while ((int)tmem_cols < bq) tmem_cols <<= 1;
+  while ((int)tmem_cols < (prm.kb_first < prm.kb_per_split ? 2 * bq : bq)) tmem_cols <<= 1;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -202,15 +204,19 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       const bool leader = elect_one();
       const uint32_t idesc = umma_idesc(2 * PR_BP, bq);
       const uint32_t lo0 = umma_desc_lo(smem_u32(smem));
-      uint32_t lo = lo0, parity = 0, accumulate = 0;
+      uint32_t lo = lo0, parity = 0, accumulate = 0, acc = tmem_base;
       int s = 0;
       for (int kb = 0; kb < num_kb; ++kb) {
         if (!warp_mbar_wait(&full_bar[s], parity, abort_flag, lane)) break;
         tc_fence_after();
+        if (kb == prm.kb_first) {
+          acc = tmem_base + (uint32_t)bq;
+          accumulate = 0;
+        }
         if (leader) {
 #pragma unroll
           for (int k = 0; k < PR_BK / 16; ++k)   // 16 bf16 = 32 bytes further along K inside the swizzled row
-            umma_bf16_pair(tmem_base, umma_desc_of(lo + 2 * k), umma_desc_of(lo + (a_bytes >> 4) + 2 * k), idesc,
+            umma_bf16_pair(acc, umma_desc_of(lo + 2 * k), umma_desc_of(lo + (a_bytes >> 4) + 2 * k), idesc,
                            k > 0 ? 1u : accumulate);
           umma_commit_pair(&empty_bar[s]);   // frees the stage, in both blocks, when these MMAs have read it
         }
@@ -258,6 +264,16 @@ linear_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         for (int sub = 0; sub < 4; ++sub)
           if (sub < n_sub) tmem_ld16_issue(lane_addr + (uint32_t)(g0 + sub * 16), raw[sub]);
         tmem_ld_wait();
+        if (second) {   // (16 columns at a time: more registers would leave room for one block an SM)
+#pragma unroll
+          for (int sub = 0; sub < 4; ++sub) {
+            if (sub >= n_sub) continue;
+            float more[16];
+            tmem_ld16(lane_addr + (uint32_t)(bq + g0 + sub * 16), more);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) raw[sub][j] = __float_as_uint(__uint_as_float(raw[sub][j]) + more[j]);
+          }
+        }
 #pragma unroll
         for (int sub = 0; sub < 4; ++sub) {
           if (sub >= n_sub) continue;
@@ -414,20 +430,26 @@ extern "C" int nib_linear_tc_pair(int out_dtype, const void* a, int lda, const v
           cost = (double)(rounds - 1) * (2.0 * kb * per_kb + fixed) +
                  (last_single ? kb * per_kb + fixed : 2.0 * kb * per_kb + fixed);
         }
-        // (ties, where twice the splits are two blocks an SM instead of one: fewer, whose tiles are added to memory less
-        // often; 2048 x 768 x 3072 in two splits 13.5 us, in four 15.6; 2048 x 1600 x 6400 in one 33.9, in two 36.1)
-        if (cost < best * 0.9999) { best = cost; best_bq = cand; best_sp = sp; }
+        if (cost < best * (sp > 1 ? 1.0001 : 1.0)) { best = cost; best_bq = cand; best_sp = sp; }   // ties: more splits
       }
     }
     bq = best_bq;
     splits = best_sp;
   }
+  // Two splits of a tile that share an SM are one block with two accumulators: the same chains of MMAs (as long a chain
+  // again would lose as much again: errors against 64 bits of 0.6e-6 and 1.2e-6 of a product, K = 3072), their sum
+  // made in registers and added to memory half as often.  2048 x 768 x 3072 as four splits 15.6 us, as two of two 13.7; 2048
+  // x 1600 x 6400 as two 36.1, as one of two 35.1.
+  const long all_blocks = 2L * pairs * ((N + bq - 1) / bq) * splits;
+  const bool merge = pick_splits && splits > 1 && all_blocks > 148 && all_blocks <= 296 && (size_t)PR_BP * bq * esz <= 100 * 1024;
+  if (merge) splits /= 2;
   if (bq < 32 || bq > 256 || bq % 32 != 0) return NIB_ERR_BAD_ARGUMENT;
   if (splits < 1 || (splits > 1 && !residual)) return NIB_ERR_BAD_ARGUMENT;
   PairParams prm;
   prm.M = M; prm.N = N; prm.K = K; prm.bq = bq;
   prm.kb_per_split = (num_kb + splits - 1) / splits;
   splits = (num_kb + prm.kb_per_split - 1) / prm.kb_per_split;
+  prm.kb_first = merge ? (prm.kb_per_split + 1) / 2 : prm.kb_per_split;
   prm.out_f32 = out_dtype == DT_F32; prm.bias = bias; prm.residual = residual; prm.status = status;
   prm.kv_cache = (bf16*)cache; prm.kv_block_table = block_table; prm.kv_row_entry = row_entry;
   prm.kv_positions = positions; prm.kv_max_blocks = max_blocks; prm.kv_q_dim = q_dim; prm.kv_heads = n_kv_head;

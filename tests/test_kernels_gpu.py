@@ -772,6 +772,37 @@ def test_product_by_pairs_of_blocks(M, N, K, bq):
     assert int(o.status_word().item()) == 0
 
 
+@pytest.mark.parametrize("M, N, K, splits, first", [(2048, 1600, 6400, 1, 3200), (2000, 1592, 6344, 1, 3200),
+                                                    (2048, 768, 3072, 2, 768), (1000, 1600, 6400, 2, 1600)])
+def test_splits_that_would_share_an_sm_are_accumulators_of_one_block(M, N, K, splits, first):
+    """Where a tile's splits of K would be two blocks an SM, one block makes them in two accumulators: no chain of MMAs is
+    longer than a split's, and what leaves the block is their sum.  ``first``: values of K in a block's first
+    accumulator.  One block a tile: the bits of the two halves made by themselves, added; two blocks: these may be
+    added in either order."""
+    o = ops()
+    g = gen(M + K)
+    a = torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(N, K, generator=g) * 0.05).to(torch.bfloat16).to(DEV)
+    b = torch.randn(N, generator=g).to(DEV)
+    x = torch.randn(M, N, generator=g).to(DEV)
+    out = x.clone()
+    assert o.linear_tc_pair(a, w, b, out, M, residual=True)
+    tiles = []
+    share = K if splits == 1 else 2 * first
+    for z in range(splits):
+        halves = []
+        for k0, k1 in ((z * share, z * share + first), (z * share + first, min(K, (z + 1) * share))):
+            part = torch.zeros(M, N, device=DEV)
+            assert o.linear_tc_pair(a[:, k0:k1], w[:, k0:k1], None, part, M, splits=1)
+            halves.append(part)
+        tiles.append(halves[0] + halves[1] + (b if z == 0 else 0.0))
+    if splits == 1:
+        assert torch.equal(out, x + tiles[0])
+    else:
+        assert bool(((out == x + tiles[0] + tiles[1]) | (out == x + tiles[1] + tiles[0])).all())
+    assert int(o.status_word().item()) == 0
+
+
 def test_product_by_pairs_declines_what_it_cannot_take():
     o = ops()
     a = torch.zeros(100, 64, dtype=torch.bfloat16, device=DEV)
