@@ -136,7 +136,7 @@ int nib_attention_prefill_tc(const void* q, int ldq, int T, const void* cache, v
                              const int* block_table, int max_blocks, const int* tiles, int n_tiles,
                              const int* entry_start, const int* entry_pos0, int n_head, int n_kv_head, int head_dim,
                              int page_size, int n_pages, float scale, int window, int sink, float softcap, int keep_first,
-                             const float* slopes, const float* gate, int ldg, float out_scale, int span, const float* head_scale, const float* sinks, int out32, int gate_dim, int pool, const int* pool_table, int* status,
+                             const float* slopes, const float* gate, int ldg, float out_scale, int span, const float* head_scale, const float* sinks, int out32, int gate_dim, int pool, const int* pool_table, int alone, int* status,
                              cudaStream_t stream);
 
 // Split-KV attention for single decoded tokens (float32 or bfloat16, head sizes up to 128 in steps

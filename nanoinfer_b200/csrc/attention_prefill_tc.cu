@@ -2,10 +2,11 @@
 // by tcgen05.mma with S and O in tensor memory, keys and values brought page by page by TMA.
 //
 // One block takes 128 consecutive query rows of one request and one head (head size 64) and walks the keys in tiles of
-// 128; two blocks share an SM.  Warp 0 is the TMA producer: its lanes look the tile's pages up in the request's block
-// table and load them (16 rows x 128 bytes a load; lanes 0..7 keys, lanes 8..15 values) into rings of two stages of
+// 128; two blocks share an SM, or, where few or long ones are left alone, one has it to itself with twice the buffers
+// (DEPTH 2).  Warp 0 is the TMA producer: its lanes look the tile's pages up in the request's block
+// table and load them (16 rows x 128 bytes a load; lanes 0..7 keys, lanes 8..15 values) into rings of two or four stages of
 // 128-byte-swizzled shared memory.  Warp 1 issues the MMAs: S = Q K^T (128 x 128 x 64) into tensor memory, the next
-// tile's as soon as the softmax warps hold this one's scores in registers; and, once they have written P to tensor
+// tile's (the one's after that with DEPTH 2) as soon as the softmax warps hold this one's scores in registers; and, once they have written P to tensor
 // memory as bfloat16, O += P V (128 x 64 x 128, P the operand that tensor memory holds, V read as it lies, keys down
 // the rows, as an MN-major operand).  Warps 2..5 are the softmax: a thread owns a row, so the row maximum and sum need
 // no exchange between threads.  The running maximum is only raised when a tile exceeds it by more than 2^8 (P stays
@@ -16,10 +17,12 @@
 //
 // What bounds it: the 128 x 128 exponentials of a tile take an SM 1,024 cycles, everything else of a softmax warp about
 // 500 issue slots; one warp a scheduler does these one after another, and with the start and end of a block in the
-// open.  With one block an SM (P through shared memory, scores three tiles ahead) a tile took 2,800 cycles; two blocks
-// an SM, each half as deep, fill each other's waits: 1,750.  On a B200, us before and now: 8 prompts of 1,003 rows and
-// 25 heads 120, 72; one of 8,144 rows and 12 heads 248, 156 (411, 655 TFLOP/s; the unit that makes the
-// exponentials 63 % busy); 2 x 1,024 rows and 12 heads, where a block has an SM to itself, 17.5, 18.0.
+// open.  Two blocks an SM fill each other's waits: 1,750 cycles a tile and SM; but each of them takes 3,500, and with one
+// score and one P buffer a block that is left alone takes as long.  With two of each it takes 2,700.  On a B200, us, one
+// block an SM with P through shared memory (as it was), two an SM, one with twice the buffers: 8 prompts of 1,003 rows and
+// 25 heads 120, 72, -; one of 8,144 rows and 12 heads 248, 156 (655 TFLOP/s; the unit that makes the exponentials 63 % busy), -;
+// one of 2,048 rows and 12 heads 26.0, 30.8, 24.5; 2 x 1,024 rows 17.0, 17.1, 15.5; 512 rows behind 7,600 88, 96, 84; 3 x 1,024
+// rows 22.3, 19.6, 20.4; 5 x 500 17.0, 12.2, 15.0.  Which: ops.prefill_blocks_alone.
 //
 // With EX the kernel takes the options of AttnExtras (api.h).  The softmax threads bring every score to its final
 // form first (scale, cap, distance bias, times log2(e); the cap by tanh(x) = 1 - 2 / (1 + e^2x) with the hardware's
@@ -152,25 +155,32 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
   return d;
 }
 
-constexpr int AT_STAGES = 2;     // stages of keys and of values
-constexpr int AT_KV_STAGE = AT_BN * 128;   // bytes of a stage: [128 keys][64]
-// tensor memory: scores (128 columns), P (64 columns of pairs), O (64)
-constexpr uint32_t AT_P_COL = AT_BN, AT_O_COL = AT_BN + AT_BN / 2, AT_TMEM_COLS = 256;
-constexpr size_t AT_SMEM = 16384 + 2 * AT_STAGES * AT_KV_STAGE + 1024;
+constexpr int AT_KV_STAGE = AT_BN * 128;   // bytes of a stage of keys or of values: [128 keys][64]
+// DEPTH: buffers of scores and of P in tensor memory, and how far the scores run ahead of the softmax.  One: two blocks
+// share an SM.  Two: one block an SM.
+template <int DEPTH>
+struct AtShape {
+  static constexpr int STAGES = 2 * DEPTH;   // of keys and of values
+  // tensor memory: the scores (128 columns each), then P (64 columns of pairs each), then O (64)
+  static constexpr uint32_t P_COL = DEPTH * AT_BN, O_COL = P_COL + DEPTH * (AT_BN / 2), TMEM_COLS = DEPTH * 256;
+  static constexpr size_t SMEM = 16384 + 2 * STAGES * AT_KV_STAGE + 1024;
+};
 constexpr float AT_RAISE = 8.0f; // the running maximum is raised when a tile exceeds it by more than 2^8
 
-template <bool EX>
-__global__ void __launch_bounds__(AT_THREADS, 2)
+template <bool EX, int DEPTH>
+__global__ void __launch_bounds__(AT_THREADS, DEPTH == 1 ? 2 : 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                             const AtParams prm) {
   extern __shared__ uint8_t at_smem_raw[];
   // tiles must start on a 1024-byte boundary for the 128-byte swizzle
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)at_smem_raw + 1023) & ~(uintptr_t)1023);
+  constexpr int AT_STAGES = AtShape<DEPTH>::STAGES;
+  constexpr uint32_t AT_P_COL = AtShape<DEPTH>::P_COL, AT_O_COL = AtShape<DEPTH>::O_COL, AT_TMEM_COLS = AtShape<DEPTH>::TMEM_COLS;
   uint8_t* q_s = smem;                                  // [128 rows][64]              16 KB
   uint8_t* k_s = q_s + 16384;                           // [stages][128 keys][64]
   uint8_t* v_s = k_s + AT_STAGES * AT_KV_STAGE;         // [stages][128 keys][64]
   __shared__ __align__(8) uint64_t q_full, k_full[AT_STAGES], k_empty[AT_STAGES], v_full[AT_STAGES], v_empty[AT_STAGES],
-      s_full, s_empty, p_full, o_full;
+      s_full[DEPTH], s_empty[DEPTH], p_full[DEPTH], o_full[DEPTH];
   __shared__ uint32_t tmem_base_sh;
   __shared__ int abort_sh;
   volatile int* abort_flag = &abort_sh;
@@ -204,10 +214,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 1);
     }
-    mbar_init(&s_full, 1);
-    mbar_init(&s_empty, 128);
-    mbar_init(&p_full, 128);
-    mbar_init(&o_full, 1);
+    for (int i = 0; i < DEPTH; ++i) {
+      mbar_init(&s_full[i], 1);
+      mbar_init(&s_empty[i], 128);
+      mbar_init(&p_full[i], 128);
+      mbar_init(&o_full[i], 1);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(&tmem_base_sh, AT_TMEM_COLS);
@@ -280,31 +292,34 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (leader) {
 #pragma unroll
         for (int k = 0; k < AT_HD / 16; ++k)   // 16 of the head's 64 values per instruction: 32 bytes along the row
-          umma_bf16(tmem_base, umma_desc_of(q_lo + 2 * k), umma_desc_of(k_lo + st * (AT_KV_STAGE / 16) + 2 * k), idesc_s, k > 0);
-        umma_commit(&s_full);
+          umma_bf16(tmem_base + (uint32_t)(it % DEPTH * AT_BN), umma_desc_of(q_lo + 2 * k), umma_desc_of(k_lo + st * (AT_KV_STAGE / 16) + 2 * k), idesc_s, k > 0);
+        umma_commit(&s_full[it % DEPTH]);
         umma_commit(&k_empty[st]);
       }
       __syncwarp();
       return true;
     };
     bool ok = warp_mbar_wait(&q_full, 0, abort_flag, lane);
-    if (ok) ok = issue_s(0);
+#pragma unroll
+    for (int a = 0; a < DEPTH; ++a)
+      if (ok && a < n_it) ok = issue_s(a);
     for (int it = 0; ok && it < n_it; ++it) {
       const int st = it % AT_STAGES;
-      if (it + 1 < n_it) {
-        if (!warp_mbar_wait(&s_empty, it & 1, abort_flag, lane)) break;   // the scores are in the softmax threads' registers
+      const int b = it % DEPTH, phase = (it / DEPTH) & 1;
+      if (it + DEPTH < n_it) {
+        if (!warp_mbar_wait(&s_empty[b], phase, abort_flag, lane)) break;   // the scores are in the softmax threads' registers
         tc_fence_after();
-        if (!issue_s(it + 1)) break;
+        if (!issue_s(it + DEPTH)) break;
       }
       if (!warp_mbar_wait(&v_full[st], (it / AT_STAGES) & 1, abort_flag, lane)) break;
-      if (!warp_mbar_wait(&p_full, it & 1, abort_flag, lane)) break;
+      if (!warp_mbar_wait(&p_full[b], phase, abort_flag, lane)) break;
       tc_fence_after();
       if (leader) {
 #pragma unroll
         for (int k = 0; k < AT_BN / 16; ++k)   // 16 keys per instruction: eight columns of P, V 16 rows down
-          umma_bf16_ts(o_tmem, p_tmem + k * 8, umma_desc_of(v_lo + st * (AT_KV_STAGE / 16) + k * 128), idesc_o,
+          umma_bf16_ts(o_tmem, p_tmem + b * (AT_BN / 2) + k * 8, umma_desc_of(v_lo + st * (AT_KV_STAGE / 16) + k * 128), idesc_o,
                        (it > 0 || k > 0) ? 1u : 0u);
-        umma_commit(&o_full);
+        umma_commit(&o_full[b]);
         umma_commit(&v_empty[st]);
       }
       __syncwarp();
@@ -328,7 +343,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     float m = -INFINITY, l = 0.0f;
     bool ok = true;
     for (int it = 0; it < n_it; ++it) {
-      ok = warp_mbar_wait(&s_full, it & 1, abort_flag, lane);
+      const int b = it % DEPTH, phase = (it / DEPTH) & 1;
+      ok = warp_mbar_wait(&s_full[b], phase, abort_flag, lane);
       if (!ok) break;
       tc_fence_after();
       const int j0 = tile_of(it) * AT_BN;
@@ -336,12 +352,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                         (span > 0 && j0 < wp1 - wp1 % span);   // only these tiles need the mask
       float v[AT_BN];
 #pragma unroll
-      for (int c = 0; c < AT_BN / 32; ++c) tmem_ld32_issue(lane_addr + (uint32_t)(c * 32), v + c * 32);
+      for (int c = 0; c < AT_BN / 32; ++c) tmem_ld32_issue(lane_addr + (uint32_t)(b * AT_BN + c * 32), v + c * 32);
       tmem_ld_wait();
 #pragma unroll
       for (int c = 0; c < AT_BN / 32; ++c) tmem_ld32_ready(v + c * 32);
       tc_fence_before();
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&s_empty)) : "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&s_empty[b])) : "memory");
       if (EX) {
         const float far = (float)(p - j0);
         if (cap_in > 0.0f) {
@@ -377,7 +393,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           const float corr = (m_new == -INFINITY) ? 1.0f : at_pow2(m - m_new);
           l *= corr;
           // O holds the tiles up to it - 1 once their MMAs are done
-          ok = warp_mbar_wait(&o_full, (it - 1) & 1, abort_flag, lane);
+          ok = warp_mbar_wait(&o_full[(it - 1) % DEPTH], ((it - 1) / DEPTH) & 1, abort_flag, lane);
           if (!ok) break;
           tc_fence_after();
 #pragma unroll 1
@@ -393,9 +409,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       }
       // a row with no key yet (all masked so far) keeps m = -inf; 2^(-inf - -inf) is avoided
       const float ms = (m == -INFINITY) ? 0.0f : m;
-      // P of the tile before has been read by its MMA
-      if (it > 0) {
-        ok = warp_mbar_wait(&o_full, (it - 1) & 1, abort_flag, lane);
+      // what this buffer of P held has been read by its MMA
+      if (it >= DEPTH) {
+        ok = warp_mbar_wait(&o_full[b], phase ^ 1, abort_flag, lane);
         if (!ok) break;
         tc_fence_after();
       }
@@ -415,7 +431,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           pk[i] = pack_bf16(e0, e1);
           pk[i + 1] = pack_bf16(e2, e3);
         }
-        tmem_st16(lane_addr + AT_P_COL + (uint32_t)(c * 16), pk);
+        tmem_st16(lane_addr + AT_P_COL + (uint32_t)(b * (AT_BN / 2) + c * 16), pk);
       }
       float s0, s1, s2, s3;
       f32x2_split(sum_a, s0, s1);
@@ -423,10 +439,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       l += (s0 + s1) + (s2 + s3);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&p_full)) : "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&p_full[b])) : "memory");
     }
     // the last MMA into O
-    if (ok) ok = warp_mbar_wait(&o_full, (n_it - 1) & 1, abort_flag, lane);
+    if (ok) ok = warp_mbar_wait(&o_full[(n_it - 1) % DEPTH], ((n_it - 1) / DEPTH) & 1, abort_flag, lane);
     if (ok) {
       tc_fence_after();
       // (the sink's term is exp(0) unless the heads have logits of their own)
@@ -472,20 +488,31 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
 using namespace nib;
 
+template <bool EX, int DEPTH>
+static int launch_at(const CUtensorMap& map_q, const CUtensorMap& map_kv, const AtParams& prm, int n_head, int n_tiles,
+                     cudaStream_t stream) {
+  auto kernel = attention_prefill_tc_kernel<EX, DEPTH>;
+  static const cudaError_t allowed =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AtShape<DEPTH>::SMEM);
+  if (allowed != cudaSuccess) return (int)allowed;
+  launch_pdl(kernel, dim3(n_head, n_tiles), dim3(AT_THREADS), AtShape<DEPTH>::SMEM, stream, map_q, map_kv, prm);
+  NIB_LAUNCH_CHECK();
+}
+
 // 1 if the tcgen05 prefill attention takes this shape (else the warp-level MMA kernel does).
 extern "C" int nib_attention_prefill_tc_supported(int head_dim, int page_size) {
   return head_dim == AT_HD && page_size >= AT_UNIT && page_size % AT_UNIT == 0;
 }
 
 // tiles: n_tiles pairs (entry, first row within the entry), 128 rows each (the last of an entry may be
-// shorter).  q [T, ldq] holds the queries of the step's T rows in its first n_head * 64 columns; cache
+// shorter).  alone: one block an SM with twice the buffers (the same results).  q [T, ldq] holds the queries of the step's T rows in its first n_head * 64 columns; cache
 // is one layer [n_pages, 2, n_kv_head, page_size, 64]; out rows must be 16-byte aligned.
 extern "C" int nib_attention_prefill_tc(const void* q, int ldq, int T, const void* cache, void* out, int ldo,
                                         const int* block_table, int max_blocks, const int* tiles, int n_tiles,
                                         const int* entry_start, const int* entry_pos0, int n_head, int n_kv_head,
                                         int head_dim, int page_size, int n_pages, float scale, int window,
                                         int sink, float softcap, int keep_first, const float* slopes, const float* gate,
-                                        int ldg, float out_scale, int span, const float* head_scale, const float* sinks, int out32, int gate_dim, int pool, const int* pool_table, int* status, cudaStream_t stream) {
+                                        int ldg, float out_scale, int span, const float* head_scale, const float* sinks, int out32, int gate_dim, int pool, const int* pool_table, int alone, int* status, cudaStream_t stream) {
   if (n_tiles <= 0) return 0;
   if (gate_dim > 0 || pool > 0) return NIB_ERR_UNSUPPORTED_SIZE;   // (attention_wide_tc.cu takes those)
   if (softcap < 0.0f || keep_first < 0) return NIB_ERR_BAD_ARGUMENT;
@@ -508,21 +535,9 @@ extern "C" int nib_attention_prefill_tc(const void* q, int ldq, int T, const voi
   prm.n_head = n_head; prm.n_kv_head = n_kv_head; prm.page_size = page_size; prm.n_pages = n_pages;
   prm.scale = scale; prm.window = window; prm.sink = sink; prm.out = (bf16*)out; prm.ldo = ldo; prm.status = status;
   prm.ex = AttnExtras{softcap, keep_first, slopes, gate, ldg, out_scale, span, head_scale, sinks, out32, gate_dim, pool, pool_table};
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)AT_SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attention_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
-  if (plain)
-    launch_pdl(attention_prefill_tc_kernel<false>, dim3(n_head, n_tiles), dim3(AT_THREADS), AT_SMEM, stream,
-               map_q, map_kv, prm);
-  else
-    launch_pdl(attention_prefill_tc_kernel<true>, dim3(n_head, n_tiles), dim3(AT_THREADS), AT_SMEM, stream,
-               map_q, map_kv, prm);
-  NIB_LAUNCH_CHECK();
+  if (plain && alone) return launch_at<false, 2>(map_q, map_kv, prm, n_head, n_tiles, stream);
+  if (plain) return launch_at<false, 1>(map_q, map_kv, prm, n_head, n_tiles, stream);
+  if (alone) return launch_at<true, 2>(map_q, map_kv, prm, n_head, n_tiles, stream);
+  return launch_at<true, 1>(map_q, map_kv, prm, n_head, n_tiles, stream);
 }
 

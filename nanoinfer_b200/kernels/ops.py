@@ -61,7 +61,7 @@ _SIGNATURES = {
     "nib_attention_prefill_tc": [_c_ptr, _c_int, _c_int, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr,
                                  _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_float, _c_int,
                                  _c_ptr, _c_ptr, _c_int, _c_float, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr,
-                           _c_ptr, _c_ptr],
+                                 _c_int, _c_ptr, _c_ptr],
     "nib_attention_simt": [_c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr,
                            _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_float, _c_int,
                            _c_ptr, _c_ptr, _c_int, _c_float, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr,
@@ -919,12 +919,26 @@ def attention_decode(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, bl
                                           _ptr(counters), _ptr(status), _stream()), "attention_decode")
 
 
+def prefill_blocks_alone(n_head: int, n_tiles: int, total: int, longest: int) -> bool:
+    """Whether the blocks of the tcgen05 prefill attention each get an SM to themselves, with twice the buffers, or share
+    one by two.  ``total``: key tiles that the ``n_tiles`` row tiles walk, ``longest``: the most that one walks.  Up to a
+    block an SM always (5 to 20 % faster there).  Beyond, in units of a lone block's key tile (1.4 us): alone the SMs are
+    busy for their share of all tiles and three more a block (its start and end stand in the open); by two the longest
+    block takes 1.3 times as long and one and a half more, and ends last.  Measured, us, alone and by two (the two sides of
+    the rule): 12 heads, 2,048 rows 24.5, 30.8 (14.9 < 22.3); 3,000 rows 39.2, 45.7 (30.2 < 32.7); 25 heads, 1,280 rows 20.7, 21.1
+    (14.4 < 14.5); 16 heads, 2 x 1,024 rows 18.6, 17.6 (13.0 > 11.9); 12 heads, 3 x 1,024 rows 20.4, 19.6 (14.6 > 11.9); 5 x 400
+    rows behind 0 to 500 19.1, 16.8 (11.92 > 11.90); 4,096 rows 70.6, 58.2 (50.6 > 43.1); 5 x 500 rows 15.0, 12.2 (8.9 > 6.7)."""
+    blocks = n_head * n_tiles
+    return blocks <= 148 or 10 * (n_head * total + 3 * blocks) <= 148 * (13 * longest + 15)
+
+
 def attention_prefill_tc(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, block_table: torch.Tensor,
                          tiles: torch.Tensor, n_tiles: int, entry_start: torch.Tensor, entry_pos0: torch.Tensor,
                          n_rows: int, n_head: int, scale: float, window: int, status: torch.Tensor,
-                         sink: bool = False, extras: Optional[AttnExtras] = None) -> None:
+                         sink: bool = False, extras: Optional[AttnExtras] = None, alone: Optional[bool] = None) -> None:
     """tcgen05 attention for prompt portions (bfloat16, head size 64): ``tiles`` holds (entry, first
-    row within the entry) pairs of 128 rows each; ``q`` holds the step's ``n_rows`` rows."""
+    row within the entry) pairs of 128 rows each; ``q`` holds the step's ``n_rows`` rows.  ``alone``: a block an SM
+    (None: up to 148 blocks); the results are the same."""
     n_pages, _, n_kv_head, page_size, head_dim = cache.shape
     if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or not _attn_out_ok(out, q.dtype, extras):
         raise KernelError("attention_prefill_tc: bfloat16 only")
@@ -934,8 +948,9 @@ def attention_prefill_tc(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor
                                               _ptr(block_table), block_table.shape[1], _ptr(tiles), n_tiles,
                                               _ptr(entry_start), _ptr(entry_pos0), n_head, n_kv_head, head_dim,
                                               page_size, n_pages, float(scale), int(window), int(sink),
-                                              *(extras or _NO_EXTRAS).args(), _ptr(status), _stream()),
-           "attention_prefill_tc")
+                                              *(extras or _NO_EXTRAS).args(),
+                                              int(n_head * n_tiles <= 148 if alone is None else alone), _ptr(status),
+                                              _stream()), "attention_prefill_tc")
 
 
 def attention_prefill(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, block_table: torch.Tensor,
@@ -1067,7 +1082,8 @@ def attention(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, block_tab
                 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0 \
                 and out.data_ptr() % 16 == 0:
             attention_prefill_tc(q, cache, out, block_table, plan.wide_tiles, plan.n_wide_tiles, ctx.entry_start,
-                                 ctx.entry_pos0, ctx.n_rows, n_head, scale, window, ctx.status, sink=sink, extras=extras)
+                                 ctx.entry_pos0, ctx.n_rows, n_head, scale, window, ctx.status, sink=sink, extras=extras,
+                                 alone=prefill_blocks_alone(n_head, plan.n_wide_tiles, *plan.wide_work(window)))
         elif fast_pages and q.dtype == torch.bfloat16 and scale > 0 and _can("nib_attention_prefill_supported", head_dim) \
                 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0:
             attention_prefill(q, cache, out, block_table, plan.tiles, plan.n_tiles, ctx.entry_start, ctx.entry_pos0,

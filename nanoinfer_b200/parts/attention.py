@@ -64,6 +64,10 @@ class AttentionPlan(StepPlan):
             dec.sort(key=lambda r: -context[r])
         self.n_decode, self.n_prefill_rows, self.n_tiles = len(dec), len(pre), len(tiles)
         self.n_wide_tiles = len(wide)
+        #: (first row's position, last row's position) of the tiles of 128 rows; ``wide_work`` by window
+        self._wide_rows = [(entry_pos0[e] + off, entry_pos0[e] + min(off + 128, entry_start[e + 1] - entry_start[e]) - 1)
+                           for e, off in wide]
+        self._wide_work = {}
         if for_graph:
             self.max_decode_keys = -(-self.max_decode_keys // GRAPH_KEY_BUCKET) * GRAPH_KEY_BUCKET
         # (the portions' rows are listed only beside decoded rows: alone they are the rows 0..n-1, and two
@@ -72,6 +76,14 @@ class AttentionPlan(StepPlan):
         self.words = dec + (pre if dec else []) + [v for t in tiles for v in t] + [v for t in wide for v in t]
         if device is not None:
             self.bind(torch.tensor(self.words, dtype=torch.int32, device=device) if self.words else None)
+
+    def wide_work(self, window: int) -> tuple:
+        """(all, most): tiles of 128 keys that the tiles of 128 rows walk with this window (0: none), of one head."""
+        got = self._wide_work.get(window)
+        if got is None:
+            walks = [last // 128 - (max(0, first - window + 1) if window > 0 else 0) // 128 + 1 for first, last in self._wide_rows]
+            got = self._wide_work[window] = (sum(walks), max(walks, default=0))
+        return got
 
     def graph_key(self) -> tuple:
         return (self.n_decode, self.n_listed_rows, self.n_tiles, self.n_wide_tiles, self.max_decode_keys)

@@ -23,3 +23,26 @@ def test_many_decoded_rows_are_listed_longest_context_first(n, portion):
         assert contexts == sorted(contexts, reverse=True) and plan.decode_rows.tolist() == listed
     else:
         assert listed == sorted(rows) and (plan.decode_rows is None) == (portion == 0)
+
+
+@pytest.mark.parametrize("window", [0, 1, 100, 128, 500])
+def test_work_of_the_wide_tiles_counts_the_key_tiles_that_are_walked(window):
+    lens, pos0 = [1, 300, 128, 129, 1, 2], [40, 0, 1000, 127, 0, 255]
+    starts = [sum(lens[:e]) for e in range(len(lens) + 1)]
+    walks = []
+    for n, p in zip(lens, pos0):
+        for off in range(0, n, 128) if n > 1 else ():
+            rows = range(p + off, p + min(off + 128, n))
+            walks.append(len(range(max(0, rows[0] - window + 1) // 128 if window else 0, rows[-1] // 128 + 1)))
+    plan = AttentionPlan(starts, pos0)
+    assert plan.n_wide_tiles == len(walks) and plan.wide_work(window) == (sum(walks), max(walks))
+    assert AttentionPlan([0, 1], [5]).wide_work(window) == (0, 0)
+
+
+def test_blocks_of_the_prefill_attention_are_left_alone_while_the_device_holds_them_and_where_one_is_long():
+    from nanoinfer_b200.kernels.ops import prefill_blocks_alone
+
+    assert prefill_blocks_alone(12, 12, 12, 1) and prefill_blocks_alone(1, 148, 5000, 60)   # 144 and 148 blocks
+    assert prefill_blocks_alone(12, 16, 136, 16)                                            # a triangle of 2,048 rows
+    assert not prefill_blocks_alone(12, 24, 108, 8) and not prefill_blocks_alone(12, 32, 528, 32)
+    assert not prefill_blocks_alone(25, 64, 288, 8)

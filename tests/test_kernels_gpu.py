@@ -280,6 +280,35 @@ def test_both_prefill_attention_kernels_at_head_size_64(case):
         assert (out.cpu().double()[rows] - want[rows]).abs().max() < 2e-2, kernel
 
 
+@pytest.mark.parametrize("case", [(2, 1, 64, 16, [900, 300, 129], [900, 130, 128], 0), (3, 3, 64, 32, [700, 60], [400, 60], 200),
+                                  (1, 1, 64, 16, [128, 2], [128, 2], 0), (2, 2, 64, 16, [385, 257], [385, 257], 0)])
+@pytest.mark.parametrize("options", ["plain", "sink", "cap"])
+def test_prefill_attention_gives_the_same_bits_alone_and_by_two(case, options):
+    """A block that has an SM to itself (two buffers of scores and of P, the scores two tiles ahead) and blocks that share
+    one: one to eight key tiles, whole and ragged, with and without a window; the maximum rises tile after tile."""
+    o = ops()
+    n_head, n_kv_head, hd, ps, lengths, q_lens, window = case
+    c = paged_case(torch.bfloat16, n_head, n_kv_head, hd, ps, lengths, q_lens, seed=sum(lengths))
+    ctx = Ctx(c["row_entry"], c["positions"])
+    plan = attention_plan(ctx)
+    for j in range(c["cache"].shape[0]):
+        c["cache"][j, 0] *= 1 + j % 7                       # (keys of very different sizes)
+    q = torch.cat(c["qs"]).to(torch.bfloat16).to(DEV)
+    cache, table = c["cache"].to(DEV), c["table"].to(DEV)
+    extras = o.AttnExtras(softcap=5.0) if options == "cap" else None
+    got = []
+    for alone in (True, False):
+        out = torch.zeros_like(q)
+        o.attention_prefill_tc(q, cache, out, table, plan.wide_tiles, plan.n_wide_tiles, ctx.entry_start, ctx.entry_pos0,
+                               ctx.n_rows, n_head, 0.3, window, ctx.status, sink=options == "sink", extras=extras, alone=alone)
+        got.append(out)
+    assert int(ctx.status.item()) == 0 and torch.equal(got[0], got[1]) and bool(got[0].any())
+    out = torch.zeros_like(q)
+    o.attention_prefill(q, cache, out, table, plan.tiles, plan.n_tiles, ctx.entry_start, ctx.entry_pos0, n_head, 0.3, window,
+                        ctx.status, sink=options == "sink", extras=extras)
+    assert (got[0].float() - out.float()).abs().max() < 2e-2
+
+
 DECODE_CASES = [
     # n_head, n_kv_head, head_dim, page, lengths (one single-token row each), window
     (12, 12, 64, 16, [1024, 1000, 513, 1], 0),
