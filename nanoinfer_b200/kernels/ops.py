@@ -845,6 +845,16 @@ def decode_split(n_rows: int, n_head: int, max_keys: int, resident: int = DECODE
     return chunk, max(1, -(-max_keys // chunk))
 
 
+def decode_longest_first(n_blocks: int, resident: int) -> bool:
+    """Whether unsplit rows are launched with the longest context first: where blocks come after the device is full, so
+    that it does not end on a long one.  While it holds them all at once, their order only says which blocks share an SM, and
+    the longest ones side by side are slower.  Contexts of 250 to 1,001, heads of 64, us for four steps, longest first and
+    in order: 16 heads (55 rows fill the device) 40 rows 6,480, 6,360; 55 7,030, 6,950; 56 6,670, 7,250; 64 7,090, 7,690; 12
+    heads (74) 64 rows 3,405, 3,275; 74 3,633, 3,582; 75 3,479, 3,735; 25 heads (35) 24 rows 16,230, 15,870; 32 16,810, 16,610; 36
+    16,805, 18,040; 12 heads in 32 bits 64 rows 11,420, 11,300; 75 12,090, 12,500; 100 13,450, 15,220."""
+    return n_blocks > resident
+
+
 def _note_attention(n_q: int, keys_seen: float, kv_rows: float, n_head: int, n_kv_head: int, head_dim: int,
                     itemsize: int, sizes=None, out_bytes: int = 0) -> None:
     """[queries, keys seen by them in all, width]: per key and head the score (2 hd), the softmax (~5)
@@ -871,9 +881,10 @@ def attention_decode(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, bl
                      row_entry: torch.Tensor, positions: torch.Tensor, n_rows: int, n_head: int, scale: float,
                      window: int, status: torch.Tensor, max_keys: int, workspace,
                      rows: Optional[torch.Tensor] = None, sink: bool = False,
-                     extras: Optional[AttnExtras] = None) -> None:
+                     extras: Optional[AttnExtras] = None, longest_first: Optional[torch.Tensor] = None) -> None:
     """Split-KV attention for rows that are single decoded tokens.  ``max_keys``: the longest key
-    range among them; partial results go through ``workspace``.  bfloat16 with a head size of 32, 64,
+    range among them; partial results go through ``workspace``.  ``longest_first``: the same rows as ``rows`` in another
+    order, for a launch that the device does not hold at once.  bfloat16 with a head size of 32, 64,
     96 or 128 runs on the warp-level MMA kernel, everything else (and float32, in true 32-bit
     arithmetic) on the streaming kernel."""
     n_pages, _, n_kv_head, page_size, head_dim = cache.shape
@@ -895,6 +906,8 @@ def attention_decode(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, bl
         if deep >= DECODE_DEEP_SPLITS:
             at_most = deep
     chunk, n_splits = decode_split(n_rows, n_head, max_keys, resident, at_most)
+    if longest_first is not None and decode_longest_first(n_rows * n_head, resident):
+        rows = longest_first
     scratch = counters = None
     if n_splits > 1:
         # (never more than the resident blocks: the same size every step, so that the buffers stay put)
@@ -1030,7 +1043,7 @@ def attention_group_mma(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor,
     lam, eps, mul = diff if diff is not None else (0.0, 0.0, 1.0)
     _check(library().nib_attention_group_mma(
         _ptr(q), q.stride(0), _ptr(cache), planes, _ptr(out), out.stride(0), int(out_head), _ptr(block_table),
-        block_table.shape[1], _ptr(plan.decode_rows), _ptr(ctx.row_entry), _ptr(ctx.positions), plan.n_decode, n_head, n_kv_head,
+        block_table.shape[1], _ptr(plan.rows_in_order), _ptr(ctx.row_entry), _ptr(ctx.positions), plan.n_decode, n_head, n_kv_head,
         row_dim, k_cols, v_cols, page_size, n_pages, float(scale), int(window), float(softcap), _ptr(gate),
         gate.stride(0) if gate is not None else 0, int(gate_dim), _ptr(sinks), int(pool), _ptr(pool_table), int(diff is not None), float(lam), float(eps), float(mul), _ptr(ctx.status),
         int(n_splits), _stream()), "attention_group_mma")
@@ -1064,10 +1077,11 @@ def attention(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, block_tab
                             q.element_size(), sizes, out.element_size())
         if fast_pages:
             attention_decode(q, cache, out, block_table, ctx.row_entry, ctx.positions, n_decode, n_head, scale,
-                             window, ctx.status, keys, ctx.workspace, plan.decode_rows, sink=sink, extras=extras)
+                             window, ctx.status, keys, ctx.workspace, plan.rows_in_order, sink=sink, extras=extras,
+                             longest_first=plan.longest_first)
         else:
             attention_simt(q, cache, out, block_table, ctx.row_entry, ctx.positions, n_decode, n_head, scale, window,
-                           ctx.status, plan.decode_rows, sink=sink, extras=extras)
+                           ctx.status, plan.rows_in_order, sink=sink, extras=extras)
     if n_portion:
         if traced:
             _note_attention(n_portion, plan.prefill_keys, plan.prefill_kv_rows, n_head, n_kv_head, head_dim,
@@ -1345,7 +1359,7 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, bl
                       e * (plan.n_decode * n_head * (D + kv_rank) + keys * D))
             if not attention_group_mma(q2, cache, out, kv_rank, block_table, ctx, plan, n_head, scale, window, D, kv_rank, gate=gate,
                                        sinks=sinks):
-                todo.append((plan.decode_rows, plan.n_decode))
+                todo.append((plan.rows_in_order, plan.n_decode))
         if plan.n_prefill_rows:
             if tracing():
                 keys = _latent_keys(ctx, window, False)
@@ -2222,10 +2236,11 @@ def _attention_general(q, cache, out, block_table, ctx, n_head, scale, window, p
     if single and page_size % 16 == 0 and head_dim % 8 == 0 and head_dim <= 128:
         keys = plan.max_decode_keys if window <= 0 else min(plan.max_decode_keys, window)
         attention_decode(q, cache, out, block_table, ctx.row_entry, ctx.positions, plan.n_decode, n_head, scale, window,
-                         ctx.status, keys, ctx.workspace, plan.decode_rows, sink=sink, extras=extras)
+                         ctx.status, keys, ctx.workspace, plan.rows_in_order, sink=sink, extras=extras,
+                         longest_first=plan.longest_first)
         return
     # (portions alone: all of the step's rows, those of no request among them, which the kernel leaves out)
-    rows, n = (plan.decode_rows, plan.n_decode) if single else (
+    rows, n = (plan.rows_in_order, plan.n_decode) if single else (
         plan.prefill_rows, plan.n_prefill_rows if plan.n_decode else ctx.n_rows)
     attention_simt(q, cache, out, block_table, ctx.row_entry, ctx.positions, n, n_head, scale, window, ctx.status, rows,
                    sink=sink, extras=extras)

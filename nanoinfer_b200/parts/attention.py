@@ -19,9 +19,8 @@ from ..kernels import ops
 from .base import (INIT_ONE_PLUS_NORMAL, MATRIX, VECTOR, KVCacheSpec, KVCacheView, Mixer, ParamSpec, PositionEncoding, StepContext,
                    StepLimits, StepPlan, Workspace, register_mixer)
 
-#: from this many decoded rows on the plan lists them, the longest context first: a launch of more blocks than the device
-#: holds at once (unsplit rows) then does not end on a long one (61 rows of 16 heads, contexts of 250 to 1,001: 38 -> 30 us
-#: a layer of a step)
+#: from this many decoded rows on the plan lists them with the longest context first as well, for launches of more blocks
+#: than the device holds at once (``ops.attention_decode`` takes the list for those alone)
 SORTED_DECODE_ROWS = 17
 #: a plan made for a graph rounds the longest key range of the decoded rows up to this many positions:
 #: the split of the keys then stays the same from step to step while the requests grow
@@ -32,7 +31,7 @@ class AttentionPlan(StepPlan):
     """Which rows of a step are single decoded tokens and which belong to prompt portions, and the
     portions cut into tiles of 64 and of 128 query rows, longest key range first; the same for
     every attention layer of the step.  Words: [decoded rows (many: the longest context first) | portion rows (only beside decoded rows) |
-    (entry, first row) per 64-row tile | the same per 128-row tile]."""
+    (entry, first row) per 64-row tile | the same per 128-row tile | decoded rows in order (many, beside portions)]."""
 
     def __init__(self, entry_start, entry_pos0, for_graph: bool = False, device=None):
         dec, pre, tiles = [], [], []
@@ -59,7 +58,9 @@ class AttentionPlan(StepPlan):
         # so that the short ones fill the gaps at the end
         tiles.sort(key=lambda t: -(entry_pos0[t[0]] + t[1]))
         wide.sort(key=lambda t: -(entry_pos0[t[0]] + t[1]))
+        in_order = []
         if len(dec) >= SORTED_DECODE_ROWS:
+            in_order = list(dec) if pre else []
             context = {entry_start[e]: entry_pos0[e] for e in range(len(entry_start) - 1)}
             dec.sort(key=lambda r: -context[r])
         self.n_decode, self.n_prefill_rows, self.n_tiles = len(dec), len(pre), len(tiles)
@@ -73,7 +74,7 @@ class AttentionPlan(StepPlan):
         # (the portions' rows are listed only beside decoded rows: alone they are the rows 0..n-1, and two
         # steps of portions that differ in a few tokens then have the same words' layout and one graph)
         self.n_listed_rows = len(pre) if dec else 0
-        self.words = dec + (pre if dec else []) + [v for t in tiles for v in t] + [v for t in wide for v in t]
+        self.words = dec + (pre if dec else []) + [v for t in tiles for v in t] + [v for t in wide for v in t] + in_order
         if device is not None:
             self.bind(torch.tensor(self.words, dtype=torch.int32, device=device) if self.words else None)
 
@@ -92,12 +93,17 @@ class AttentionPlan(StepPlan):
         """``buf``: a device int32 tensor holding ``self.words``."""
         nd, npre = self.n_decode, self.n_listed_rows
         all_decode = self.n_prefill_rows == 0
-        # rows 0..n-1 in order need no index list
-        self.decode_rows = None if nd == 0 or (all_decode and nd < SORTED_DECODE_ROWS) else buf[:nd]
+        many = nd >= SORTED_DECODE_ROWS
+        self.decode_rows = None if nd == 0 or (all_decode and not many) else buf[:nd]
+        #: the decoded rows with the longest context first (None: too few to be listed so)
+        self.longest_first = self.decode_rows if many else None
         self.prefill_rows = None if nd == 0 or npre == 0 else buf[nd:nd + npre]
         self.tiles = buf[nd + npre:nd + npre + 2 * self.n_tiles] if self.n_tiles else None
         at = nd + npre + 2 * self.n_tiles
         self.wide_tiles = buf[at:at + 2 * self.n_wide_tiles] if self.n_wide_tiles else None
+        at += 2 * self.n_wide_tiles
+        #: the decoded rows in order (None: they are the rows 0..n-1)
+        self.rows_in_order = None if nd == 0 or all_decode else buf[at:at + nd] if many else buf[:nd]
 
 
 def _split(xn):
