@@ -252,9 +252,9 @@ def time_prefill(eng, n_prompts: int, prompt_len: int, runs: int, warmup: int, s
         reqs = [eng.cache.open_request() for _ in range(n_prompts)]
         items = [StepItem(r, torch.randint(0, vocab, (prompt_len,), generator=g).tolist(), [prompt_len - 1])
                  for r in reqs]
-        flusher.flush()
-        torch.cuda.synchronize()
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        flusher.flush()      # (the host packs the step meanwhile: a wait here would put that between the events)
         e0.record()
         eng.runner.step(items)
         e1.record()
