@@ -482,15 +482,26 @@ static int launch_features(const InT* a, int lda, const InT* w, int ldw, const f
 // 3.35, 16 rows 3.52, 5.58; K = 256, 16 rows 6.31, 6.05.  N = 9,600: K = 64, 8 rows 3.05, 6.76; K = 128, 1 row 4.29, 3.86, 4 rows
 // 4.39, 5.01; K = 256, 8 rows 9.32, 7.57, 16 rows 9.87, 12.34; K = 384, 16 rows 14.4, 13.6.  N = 50,257, K = 768, 16 rows 83, 86.
 // bfloat16: N = 768, K = 33: 8 rows 2.12, 3.67; K = 100: 4 rows 2.96, 2.41, 8 rows 3.00, 3.60; N = 9,600, K = 130: 8 rows 7.24, 10.07.
+// From how many features on it is ahead whatever K: the other kernel's time grows with their number, and where K takes
+// several stages it reads the rows again for every eight of them; without asynchronous copies it waits for every stage.
+// us, this one and the other, 16 rows, 32-bit: K = 768: N = 9,601 28, 20; 14,400 28, 27; 18,944 28, 35.  K = 1,600: 8,192 53, 48;
+// 12,288 58, 73; 18,944 59, 108; 50,257 173, 284.  8 rows: K = 768, 50,257 59, 49; K = 1,600: 14,400 62, 49; 18,944 45, 62; 50,257
+// 123, 161.  Odd pitches, 16 rows: K = 769: 8,192 28, 26; 9,601 30, 32; K = 1,601: 5,120 52, 47; 6,144 42, 56; 8 rows: K = 769:
+// 14,400 32, 28; 18,944 23, 36; K = 1,601: 9,601 59, 50; 12,288 57, 66; 4 rows, K = 1,601: 14,400 64, 47; 18,944 46, 60.  bfloat16, 16
+// rows: K = 769: 9,601 42, 37; 12,288 42, 46; K = 1,601: 6,144 79, 78; 7,168 82, 90; 8 rows: K = 769: 12,288 36, 33; 14,400 36, 39;
+// K = 1,601: 9,601 69, 67; 12,288 71, 87; 4 rows: behind up to 50,257.
 template <typename InT, bool VEC>
 static bool features_pay(int M, int N, int K) {
-  const bool wide = N >= 8192, middle = N >= 2048, half = sizeof(InT) == 2;
+  const bool wide = N >= 8192, middle = N >= 2048, half = sizeof(InT) == 2, stages = K > RW_K;
   int most;
   if (M <= 2) most = half && wide ? 2 : 1;
   else if (M <= 4) most = wide || (middle && (VEC || half)) ? 2 : 1;
-  else if (M <= 8) most = half ? (wide ? 3 : 2) : VEC ? (wide ? 3 : middle ? 2 : 1) : wide ? 2 : 1;
-  else most = VEC && N >= 32768 ? 12 : wide ? 5 : middle ? 3 : VEC ? 1 : 2;
-  return (K + FB_K - 1) / FB_K <= most;
+  else if (M <= 8) most = half ? (wide ? 3 : 2) : VEC ? (N >= 16384 ? 4 : wide ? 3 : middle ? 2 : 1) : wide ? 2 : 1;
+  else most = wide ? 5 : middle ? 3 : VEC ? 1 : 2;
+  if ((K + FB_K - 1) / FB_K <= most) return true;
+  if (M <= 4) return !VEC && !half && stages && N >= 16384;
+  if (M <= 8) return VEC ? stages && N >= 16384 : N >= (stages ? 12288 : half ? 14336 : 16384);
+  return N >= (VEC ? (stages ? 12288 : 16384) : half ? (stages ? 7168 : 12288) : (stages ? 6144 : 9216));
 }
 
 template <typename InT, typename OutT, int TM, bool VEC>

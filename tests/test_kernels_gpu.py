@@ -280,6 +280,29 @@ def test_both_prefill_attention_kernels_at_head_size_64(case):
         assert (out.cpu().double()[rows] - want[rows]).abs().max() < 2e-2, kernel
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N, K", [(6145, 1057), (7168, 1028), (9216, 360), (12289, 1100), (14337, 100), (16384, 1056)])
+@pytest.mark.parametrize("pad", [0, 1])
+def test_linear_of_few_rows_with_wide_outputs(N, K, pad, dtype):
+    """Outputs wide enough that a feature a thread is ahead whatever K: the bits of the kernel that takes the same rows in
+    a larger step, without and with 16-byte copies (32-bit values, K a multiple of four, no ``pad``)."""
+    g = gen(7)
+    o = ops()
+    w = torch.randn(N, K + pad, generator=g).to(dtype)[:, :K].to(DEV)
+    a = torch.randn(17, K + pad, generator=g).to(dtype)[:, :K].to(DEV)
+    bias = torch.randn(N, generator=g).to(DEV)
+    many = torch.zeros(17, N, device=DEV)
+    o.linear_simt(a, w, bias, many, 17)
+    a64, w64 = a.double(), w.double()
+    # (32 roundings of a chain, a quarter's segments, the quarters and the bias, times the sum of magnitudes)
+    bound = (32 + K // 128 + 8) * 2.0 ** -24 * (a64.abs() @ w64.abs().T + bias.double().abs())
+    assert bool(((many.double() - a64 @ w64.T - bias.double()).abs() <= bound).all())
+    for M in (2, 4, 5, 8, 9, 16):
+        few = torch.full((M + 1, N), 7.0, device=DEV)
+        o.linear_simt(a, w, bias, few, M)
+        assert torch.equal(few[:M], many[:M]) and bool((few[M] == 7.0).all()), M
+
+
 @pytest.mark.parametrize("case", [(2, 1, 64, 16, [900, 300, 129], [900, 130, 128], 0), (3, 3, 64, 32, [700, 60], [400, 60], 200),
                                   (1, 1, 64, 16, [128, 2], [128, 2], 0), (2, 2, 64, 16, [385, 257], [385, 257], 0)])
 @pytest.mark.parametrize("options", ["plain", "sink", "cap"])
