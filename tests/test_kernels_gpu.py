@@ -303,6 +303,27 @@ def test_linear_of_few_rows_with_wide_outputs(N, K, pad, dtype):
         assert torch.equal(few[:M], many[:M]) and bool((few[M] == 7.0).all()), M
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M, N, K", [(17, 65, 1), (33, 130, 31), (64, 63, 33), (65, 64, 63), (200, 9600, 35), (161, 4800, 97),
+                                     (640, 1000, 129)])
+def test_linear_in_tiles_without_asynchronous_copies(M, N, K, dtype):
+    """Segments that wait in registers: one, two and several of them, the last one value, four or all but one long, alone
+    and in a cluster of four that shares K; each row the bits of a step of its own."""
+    g = gen(8)
+    o = ops()
+    w = torch.randn(N, K + 1, generator=g).to(dtype)[:, 1:].to(DEV)
+    a = torch.randn(M, K + 1, generator=g).to(dtype)[:, 1:].to(DEV)
+    out = torch.full((M + 1, N), 7.0, device=DEV)
+    o.linear_simt(a, w, None, out, M)
+    a64, w64 = a.double(), w.double()
+    bound = (32 + K // 128 + 8) * 2.0 ** -24 * (a64.abs() @ w64.abs().T)
+    assert bool(((out[:M].double() - a64 @ w64.T).abs() <= bound).all()) and bool((out[M] == 7.0).all())
+    one = torch.zeros(1, N, device=DEV)
+    for m in (0, M // 2, M - 1):
+        o.linear_simt(a[m:m + 1], w, None, one, 1)
+        assert torch.equal(one[0], out[m]), m
+
+
 @pytest.mark.parametrize("case", [(2, 1, 64, 16, [900, 300, 129], [900, 130, 128], 0), (3, 3, 64, 32, [700, 60], [400, 60], 200),
                                   (1, 1, 64, 16, [128, 2], [128, 2], 0), (2, 2, 64, 16, [385, 257], [385, 257], 0)])
 @pytest.mark.parametrize("options", ["plain", "sink", "cap"])
