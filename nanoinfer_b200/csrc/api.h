@@ -118,6 +118,14 @@ int nib_linear_skinny(int out_dtype, const void* a, int lda, const void* w, int 
                       const int* positions, int q_dim, int n_kv_head, int head_dim, int page_size, int n_pages,
                       int split, int* status, cudaStream_t stream);
 
+// The product for steps of at most 8 rows, with the options of nib_linear_skinny but for the split.
+// NIB_ERR_UNSUPPORTED_SIZE where a size or an alignment is not taken.
+int nib_linear_few(int out_dtype, const void* a, int lda, const void* w, int ldw, const float* bias, void* out, int ldo,
+                   int M, int N, int K, int act, int residual, const float* ln_x, int ln_ldx, const float* ln_gamma,
+                   const float* ln_beta, float ln_eps, const int* ln_rows, void* cache, const int* block_table,
+                   int max_blocks, const int* row_entry, const int* positions, int q_dim, int n_kv_head, int head_dim,
+                   int page_size, int n_pages, int* status, cudaStream_t stream);
+
 // Causal attention of T query rows over the paged cache (general SIMT kernel).  rows: the
 // step's rows to process (nullptr: rows 0..T-1).  `sink` (here and in the attention kernels below): 1 adds one
 // term exp(0) to the softmax's denominator, a key of score 0 that has no value.

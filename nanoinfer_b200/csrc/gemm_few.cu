@@ -1,0 +1,520 @@
+// out = act(a . w^T + bias) for steps of one to eight rows, in bfloat16: a decode step of a few requests.
+//
+// Such a product is a stream of weights with a handful of multiply-adds each, one of a hundred dependent launches of a
+// step, and what counts is the chain from the end of the kernel ahead to its own last store.  (A launch boundary under
+// programmatic dependent launch with one dependent load and store measures 1.1 us in a graph; the kernel for up to 128
+// rows, gemm_skinny.cu, took 2.5 to 10 us between its boundaries at these sizes.)  So:
+//   * the weights of a block are whole rows and come by the copy engine (`cp.async.bulk`, one instruction a row) into
+//     shared memory, all of them asked for before the wait for the kernel ahead: they need no registers, whatever K is,
+//     and do not queue in front of the step's rows in the load path;
+//   * one block an SM (at most), each with a contiguous share of the output's tiles, so that the rows are read and
+//     normalised once per SM;
+//   * the step's rows never pass through shared memory: a lane loads the pieces of its row in the order in which the
+//     MMA (m16n8k16) wants them, and normalises them there.  The statistics of a row are merged from one mean and one
+//     sum of squared differences per warp, with a single barrier;
+//   * K is not split over blocks: eight warps split it, and their sums meet in shared memory once.
+// F = 16: a tile is 16 features, weights are the MMA's 16-row operand.  F = 8: a tile is 8 features, the step's rows are
+// the 16-row operand (half of it zeros); twice the MMAs a weight, but a narrow output still reaches twice as many SMs.
+//
+// Folded in, as in gemm_skinny.cu: the norm before the product, bias, GELU and residual, and the write of keys and
+// values into the paged cache.  A row's result does not depend on the rows beside it.
+//
+// Measured (B200; in a graph, weights from memory; us a launch of the four products of a layer and their mean in the
+// order of a step; gemm_skinny.cu before, this now):
+//   GPT-2 small, 8 rows  q/k/v 3.9, 3.2   output 2.5, 2.05  MLP 4.2, 2.9   4.2, 3.1   mean 3.5, 3.0
+//   GPT-2 XL, 8 rows           9.6, 5.9          4.1, 2.6       10.0, 6.8  8.5, 6.0        7.4, 5.0
+// Whole decode steps: small 231 -> 196 us at one row, 309 -> 262 at eight, XL 1,915 -> 1,556 at eight (perf/cases.py).
+// What is left at 8 rows of small: 0.5 us launch, 0.3 for the stores to be visible, about 0.4 until the rows are here,
+// 0.45 statistics and normalisation, 0.25 MMAs, 0.3 sums across warps and epilogue; at XL's sizes the weights' way into
+// shared memory (104 to 205 KB an SM).
+#include "api.h"
+#include "tcgen05.cuh"
+
+namespace nib {
+
+constexpr int FW_WARPS = 8;
+constexpr int FW_ROWS = 8;            // rows of a step, at most
+constexpr int FW_SMS = 148;
+constexpr int FW_MAX_BARS = 16;       // groups of tiles in flight, at most
+constexpr int FW_RED_PITCH = 20;      // floats between the rows of a tile's partial sums (16 features): no bank conflicts
+constexpr size_t FW_SMEM_LIMIT = 220 * 1024;
+
+struct FewParams {
+  const bf16* a;        // [M, K] activations (LN: unused)
+  int lda;
+  const float* ln_x;    // LN: the residual stream, normalised here
+  int ln_ldx;
+  const float* ln_gamma;
+  const float* ln_beta;   // null: an RMS norm (nothing is taken off, nothing added)
+  const int* ln_rows;
+  float ln_eps;
+  const bf16* w;        // [N, K]
+  int ldw;
+  const float* bias;
+  void* out;
+  int ldo, out_f32, residual, act;
+  int M, N, K;
+  int stages;           // groups of tiles in flight
+  int per_block, wide;  // tiles a block, and how many blocks have one more
+  float inv_k;          // 1 / K
+  bf16* kv_cache;       // optional: features from kv_q_dim on go to the paged cache
+  const int* kv_block_table;
+  const int* kv_row_entry;
+  const int* kv_positions;
+  int kv_max_blocks, kv_q_dim, kv_heads, kv_head_dim, kv_page_size, kv_n_pages;
+  int* status;
+};
+
+__device__ __forceinline__ void few_mma(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t few_pack(float lo, float hi) {
+  __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
+// one row of weights, `bytes` (a multiple of 16), both addresses on 16 bytes
+__device__ __forceinline__ void few_bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+// elements between the weight rows of a tile: pieces of 8 rows x 4 lanes hit distinct banks
+__host__ __device__ inline int few_pitch(int K) { return K + ((32 - K % 64) + 64) % 64; }
+
+// two 32-bit values in one register pair
+__device__ __forceinline__ uint64_t two(float lo, float hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ void split2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint32_t pack2x(uint64_t v) {
+  float lo, hi;
+  split2(v, lo, hi);
+  return few_pack(lo, hi);
+}
+// 1 / sqrt(v) for v > 0: the hardware's estimate and one Newton step (a division and a root by the library are calls of
+// 60 and 140 cycles, more where a lane's value is zero, in the middle of a chain of about 3,000)
+__device__ __forceinline__ float few_rsqrt(float v) {
+  const float y = rsqrtf(v);
+  const float z = fmaf(0.5f * y, fmaf(-v * y, y, 1.0f), y);
+  return v < 3.0e38f ? z : y;      // (an overflowed variance: 0, as 1 / sqrt(inf))
+}
+
+// GT: tiles of a group (their sums are added up behind one barrier); ST: 32-wide steps of K a warp has (K <= 256 * ST);
+// warp w takes the steps w, w + 8, ...
+template <int F, int GT, int ST, bool LN>
+__global__ void __launch_bounds__(FW_WARPS * 32, 2) linear_few_kernel(const __grid_constant__ FewParams prm) {
+  pdl_trigger();
+  constexpr int R = LN || ST <= 8 ? ST : 8;                // steps of the row that a lane holds at a time
+  constexpr int CH = F == 16 ? (GT == 1 ? 2 : 1) : (GT == 1 ? 4 : 2);   // independent chains of MMAs a tile
+  constexpr int TILE_SUMS = FW_ROWS * F;
+  constexpr int OUTS = (GT * TILE_SUMS + FW_WARPS * 32 - 1) / (FW_WARPS * 32);
+  extern __shared__ __align__(128) uint8_t fw_smem[];
+  __shared__ __align__(8) uint64_t bars[FW_MAX_BARS];
+  __shared__ float4 stats[FW_WARPS][FW_ROWS];
+  __shared__ int abort_sh;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31, fr = lane >> 2, kl = lane & 3;
+  const int M = prm.M, N = prm.N, K = prm.K, n_chunks = K >> 3;
+  const int pitch = few_pitch(K);
+  // this block's tiles: the first `wide` blocks have one more
+  const int t_begin = blockIdx.x * prm.per_block + min((int)blockIdx.x, prm.wide);
+  const int mine = prm.per_block + ((int)blockIdx.x < prm.wide ? 1 : 0);
+  const int groups = (mine + GT - 1) / GT, S = prm.stages;
+  bf16* ws = reinterpret_cast<bf16*>(fw_smem);             // [stages][GT][F][pitch]
+  float* red = reinterpret_cast<float*>(fw_smem + (size_t)S * GT * F * pitch * sizeof(bf16));
+  constexpr int RED = FW_WARPS * GT * FW_ROWS * FW_RED_PITCH;   // [2][warps][GT][rows][pitch]
+  float* gb = red + (S > 1 ? 2 : 1) * RED;                 // LN: [2][K] scale and shift
+
+  // ---- Before the wait: what the kernel ahead does not write.
+  if (LN) {   // (ahead of the weights: they are needed first)
+    for (int i = threadIdx.x; i < K / 4; i += FW_WARPS * 32) {
+      cp_async16(gb + i * 4, prm.ln_gamma + i * 4, true);
+      cp_async16(gb + K + i * 4, prm.ln_beta != nullptr ? prm.ln_beta + i * 4 : prm.ln_gamma, prm.ln_beta != nullptr);
+    }
+    cp_async_commit();
+  }
+  auto ask = [&](int g, int slot) {      // (the first warp) the weights of group g
+    // (a group's tiles are neighbours: one run of rows here and there)
+    const int f0 = (t_begin + g * GT) * F, rows = min(min(GT, mine - g * GT) * F, N - f0);
+    if (elect_one()) {
+      mbar_expect_tx(&bars[slot], (uint32_t)rows * K * 2);
+      const bf16* src = prm.w + (size_t)f0 * prm.ldw;
+      bf16* dst = ws + (size_t)slot * GT * F * pitch;
+      for (int r = 0; r < rows; ++r) few_bulk_load(dst + (size_t)r * pitch, src + (size_t)r * prm.ldw, (uint32_t)K * 2, &bars[slot]);
+    }
+  };
+  if (warp == 0) {
+    if (elect_one()) {
+      abort_sh = 0;
+      for (int i = 0; i < S; ++i) mbar_init(&bars[i], 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    for (int g = 0; g < S && g < groups; ++g) ask(g, g);
+  }
+  // output q of this thread within a group: tile, row and feature
+  auto place = [&](int q, int& j, int& m, int& nl) {
+    const int o = threadIdx.x + q * FW_WARPS * 32;
+    j = o / TILE_SUMS; m = (o % TILE_SUMS) / F; nl = o % F;
+    return o < GT * TILE_SUMS && m < M;
+  };
+  float bias_r[OUTS], res_r[OUTS];
+  long long kv_at[OUTS];   // where in the cache layer the output goes (-1: to `out`, -2: nowhere, -3: the page is none of the pool's)
+  auto fetch = [&](int g) {   // bias and destination of group g's outputs
+#pragma unroll
+    for (int q = 0; q < OUTS; ++q) {
+      int j, m, nl;
+      const bool ok = place(q, j, m, nl) && g * GT + j < mine;
+      const int n = (t_begin + g * GT + j) * F + nl;
+      bias_r[q] = 0.0f;
+      kv_at[q] = -1;
+      if (ok && n < N) {
+        if (prm.bias != nullptr) bias_r[q] = prm.bias[n];
+        if (prm.kv_cache != nullptr && n >= prm.kv_q_dim) {
+          const int pos = prm.kv_positions[m], entry = prm.kv_row_entry[m];
+          const int page = entry < 0 ? 0 : prm.kv_block_table[(size_t)entry * prm.kv_max_blocks + pos / prm.kv_page_size];
+          const int kv_dim = prm.kv_heads * prm.kv_head_dim, rem = n - prm.kv_q_dim, which = rem >= kv_dim ? 1 : 0;
+          const int at = rem - which * kv_dim, head = at / prm.kv_head_dim;
+          kv_at[q] = entry < 0 ? -2
+                     : (page < 0 || page >= prm.kv_n_pages)
+                         ? -3
+                         : (long long)kv_offset(page, which, head, pos % prm.kv_page_size, prm.kv_heads, prm.kv_page_size,
+                                                prm.kv_head_dim) + (at - head * prm.kv_head_dim);
+        }
+      }
+    }
+  };
+  auto fetch_residual = [&](int g) {
+#pragma unroll
+    for (int q = 0; q < OUTS; ++q) {
+      int j, m, nl;
+      const bool ok = place(q, j, m, nl) && g * GT + j < mine;
+      const int n = (t_begin + g * GT + j) * F + nl;
+      res_r[q] = 0.0f;
+      if (ok && prm.residual && n < N) res_r[q] = ((const float*)prm.out)[(size_t)m * prm.ldo + n];
+    }
+  };
+  fetch(0);
+  const bool row_here = fr < M;
+  const float* xrow = nullptr;
+  if (LN && row_here) xrow = prm.ln_x + (size_t)(prm.ln_rows ? prm.ln_rows[fr] : fr) * prm.ln_ldx;
+  float n_vals = 0.0f, inv_n = 0.0f;              // values of a row that this warp sums
+  if (LN) {
+    int n = 0;
+#pragma unroll
+    for (int s = 0; s < ST; ++s) n += 8 * max(0, min(4, n_chunks - 4 * (warp + s * FW_WARPS)));
+    n_vals = (float)n;
+    inv_n = n > 0 ? 1.0f / n_vals : 0.0f;
+  }
+  __syncthreads();             // the barriers are initialised
+  pdl_wait();
+
+  // ---- the step's rows, in the order of the MMA's operands: of step s, the eight values at (warp + 8 s) * 32 + 8 kl
+  uint4 xb[R];
+  auto load_x = [&](int s) {
+    const int c = (warp + s * FW_WARPS) * 4 + kl;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (row_here && c < n_chunks) v = *reinterpret_cast<const uint4*>(prm.a + (size_t)fr * prm.lda + c * 8);
+    return v;
+  };
+  if (!LN) {
+#pragma unroll
+    for (int s = 0; s < R; ++s) xb[s] = load_x(s);
+  }
+  if constexpr (LN) {
+    uint64_t xf[ST][4];        // pairs of neighbours
+#pragma unroll
+    for (int s = 0; s < ST; ++s) {
+      const int c = (warp + s * FW_WARPS) * 4 + kl;
+      ulonglong2 lo = make_ulonglong2(0, 0), hi = lo;
+      if (row_here && c < n_chunks) {
+        lo = *reinterpret_cast<const ulonglong2*>(xrow + c * 8);
+        hi = *reinterpret_cast<const ulonglong2*>(xrow + c * 8 + 4);
+      }
+      xf[s][0] = lo.x; xf[s][1] = lo.y; xf[s][2] = hi.x; xf[s][3] = hi.y;
+    }
+    // this warp's sum and its squared differences from its own mean; then all warps' merged (an RMS norm: mean 0)
+    const bool shifted = prm.ln_beta != nullptr;
+    uint64_t s2 = 0;
+#pragma unroll
+    for (int s = 0; s < ST; ++s) s2 = add2(s2, add2(add2(xf[s][0], xf[s][1]), add2(xf[s][2], xf[s][3])));
+    float sum, sum_hi;
+    split2(s2, sum, sum_hi);
+    sum += sum_hi;
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    const float own = shifted ? sum * inv_n : 0.0f;
+    uint64_t q2 = 0;
+#pragma unroll
+    for (int s = 0; s < ST; ++s) {
+      const float c0 = (warp + s * FW_WARPS) * 4 + kl < n_chunks ? -own : 0.0f;   // (zeros past the row)
+      const uint64_t cc = two(c0, c0);
+      const uint64_t d0 = add2(xf[s][0], cc), d1 = add2(xf[s][1], cc), d2 = add2(xf[s][2], cc), d3 = add2(xf[s][3], cc);
+      q2 = add2(q2, add2(fma2(d0, d0, mul2(d1, d1)), fma2(d2, d2, mul2(d3, d3))));
+    }
+    float sq, sq_hi;
+    split2(q2, sq, sq_hi);
+    sq += sq_hi;
+    sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+    sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+    if (kl == 0) stats[warp][fr] = make_float4(sum, sq, own, n_vals);
+    cp_async_wait<0>();        // (the norm's parameters)
+    __syncthreads();
+    float total = 0.0f, squares = 0.0f;
+    float4 st[FW_WARPS];
+#pragma unroll
+    for (int w = 0; w < FW_WARPS; ++w) { st[w] = stats[w][fr]; total += st[w].x; }
+    const float mean = shifted ? total * prm.inv_k : 0.0f;
+#pragma unroll
+    for (int w = 0; w < FW_WARPS; ++w) { const float d = st[w].z - mean; squares += st[w].y + st[w].w * d * d; }
+    const float rstd = few_rsqrt(squares * prm.inv_k + prm.ln_eps);
+    const uint64_t mm = two(-mean, -mean), rr = two(rstd, rstd);
+#pragma unroll
+    for (int s = 0; s < ST; ++s) {
+      const int cc = (warp + s * FW_WARPS) * 4 + kl;
+      const bool ok = row_here && cc < n_chunks;
+      const int c = cc < n_chunks ? cc : 0;      // (no branch: the steps' chains run side by side)
+      {
+        const ulonglong2 g0 = *reinterpret_cast<const ulonglong2*>(gb + c * 8), g1 = *reinterpret_cast<const ulonglong2*>(gb + c * 8 + 4);
+        const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(gb + K + c * 8), b1 = *reinterpret_cast<const ulonglong2*>(gb + K + c * 8 + 4);
+        xb[s].x = ok ? pack2x(fma2(mul2(add2(xf[s][0], mm), rr), g0.x, b0.x)) : 0u;
+        xb[s].y = ok ? pack2x(fma2(mul2(add2(xf[s][1], mm), rr), g0.y, b0.y)) : 0u;
+        xb[s].z = ok ? pack2x(fma2(mul2(add2(xf[s][2], mm), rr), g1.x, b1.x)) : 0u;
+        xb[s].w = ok ? pack2x(fma2(mul2(add2(xf[s][3], mm), rr), g1.y, b1.y)) : 0u;
+      }
+    }
+  }
+  fetch_residual(0);
+
+  volatile int* abort_flag = &abort_sh;
+  int slot = 0, round = 0;     // g % S, g / S
+#pragma unroll 1
+  for (int g = 0; g < groups; ++g) {
+    if (g > 0) {
+      fetch(g);
+      fetch_residual(g);
+      if (R < ST) {
+#pragma unroll
+        for (int s = 0; s < R; ++s) xb[s] = load_x(s);
+      }
+    }
+    float acc[GT][CH][4];
+#pragma unroll
+    for (int j = 0; j < GT; ++j)
+#pragma unroll
+      for (int c = 0; c < CH; ++c) acc[j][c][0] = acc[j][c][1] = acc[j][c][2] = acc[j][c][3] = 0.0f;
+    const bf16* w0 = ws + ((size_t)slot * GT * F + fr) * pitch;
+    mbar_wait(&bars[slot], round & 1, abort_flag);
+#pragma unroll
+    for (int s = 0; s < ST; ++s) {
+      const int c = (warp + s * FW_WARPS) * 4 + kl;
+      const uint4 x = xb[s % R];
+      if (R < ST && s + R < ST) xb[s % R] = load_x(s + R);
+#pragma unroll
+      for (int j = 0; j < GT; ++j) {
+        // (past the row, and of a tile that this block does not have: zeros, not what the memory held)
+        uint4 wa = make_uint4(0, 0, 0, 0), wb = wa;
+        if (c < n_chunks && (j == 0 || g * GT + j < mine)) {
+          wa = *reinterpret_cast<const uint4*>(w0 + (size_t)j * F * pitch + c * 8);
+          if (F == 16) wb = *reinterpret_cast<const uint4*>(w0 + ((size_t)j * F + 8) * pitch + c * 8);
+        }
+        float* d = acc[j][s % CH];
+        if (F == 16) {
+          few_mma(d, wa.x, wb.x, wa.y, wb.y, x.x, x.y);
+          few_mma(d, wa.z, wb.z, wa.w, wb.w, x.z, x.w);
+        } else {
+          few_mma(d, x.x, 0, x.y, 0, wa.x, wa.y);
+          few_mma(d, x.z, 0, x.w, 0, wa.z, wa.w);
+        }
+      }
+    }
+    // ---- the warps' sums meet in shared memory, [row][feature]
+    float* rd = red + (S > 1 ? (g & 1) * RED : 0);
+#pragma unroll
+    for (int j = 0; j < GT; ++j) {
+      float* r0 = rd + (warp * GT + j) * FW_ROWS * FW_RED_PITCH;
+      float* d = acc[j][0];
+#pragma unroll
+      for (int c = 1; c < CH; ++c)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d[e] += acc[j][c][e];
+      if (F == 16) {     // a lane has features fr and fr + 8 of rows 2 kl and 2 kl + 1
+        r0[(2 * kl) * FW_RED_PITCH + fr] = d[0];
+        r0[(2 * kl + 1) * FW_RED_PITCH + fr] = d[1];
+        r0[(2 * kl) * FW_RED_PITCH + fr + 8] = d[2];
+        r0[(2 * kl + 1) * FW_RED_PITCH + fr + 8] = d[3];
+      } else {           // features 2 kl and 2 kl + 1 of row fr
+        *reinterpret_cast<float2*>(r0 + fr * FW_RED_PITCH + 2 * kl) = make_float2(d[0], d[1]);
+      }
+    }
+    __syncthreads();
+    if (S > 1 && warp == 0 && g + S < groups) ask(g + S, slot);   // every warp has read this group's weights
+#pragma unroll
+    for (int q = 0; q < OUTS; ++q) {
+      int j, m, nl;
+      const bool ok = place(q, j, m, nl) && g * GT + j < mine;
+      const int n = (t_begin + g * GT + j) * F + nl;
+      if (!ok || n >= N) continue;
+      float p[FW_WARPS];
+#pragma unroll
+      for (int w = 0; w < FW_WARPS; ++w) p[w] = rd[((w * GT + j) * FW_ROWS + m) * FW_RED_PITCH + nl];
+      float x = ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7])) + bias_r[q];
+      if (prm.act == ACT_GELU_TANH) {
+        float th;
+        asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(0.7978845608028654f * (x + 0.044715f * x * x * x)));
+        x = 0.5f * x * (1.0f + th);
+      } else if (prm.act == ACT_GELU_ERF) {
+        x = gelu_erf(x);
+      } else if (prm.act == ACT_RELU_SQ) {
+        x = relu_sq(x);
+      }
+      if (kv_at[q] != -1) {
+        if (kv_at[q] == -3)
+          *prm.status = NIB_STATUS_BAD_PAGE;
+        else if (kv_at[q] >= 0)
+          prm.kv_cache[kv_at[q]] = __float2bfloat16_rn(x);
+      } else if (prm.out_f32) {
+        ((float*)prm.out)[(size_t)m * prm.ldo + n] = prm.residual ? res_r[q] + x : x;
+      } else {
+        ((bf16*)prm.out)[(size_t)m * prm.ldo + n] = __float2bfloat16_rn(x);
+      }
+    }
+    if (++slot == S) { slot = 0; ++round; }
+  }
+  if (abort_sh) {   // a copy did not come in time: no thread leaves while one may still be under way
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      *prm.status = NIB_STATUS_WAIT_TIMEOUT;
+      const long long t0 = clock64();
+      for (int i = 0; i < S && i < groups; ++i)
+        while (!mbar_try_wait(&bars[i], ((groups - 1 - i) / S) & 1) && clock64() - t0 < TC_WAIT_CYCLES) {}
+    }
+    __syncthreads();
+  }
+}
+
+// How a product is cut: F features a tile, GT tiles a group, ST steps a warp, stages of groups in flight.
+struct FewPlan { int F, GT, ST, stages, blocks; size_t smem; };
+
+static bool few_plan(int M, int N, int K, bool ln, FewPlan& p) {
+  if (M < 1 || M > FW_ROWS || N < 1 || K < 8 || (K & 7)) return false;
+  const int st = (K + 255) / 256;
+  p.ST = st <= 3 ? 3 : st <= 4 ? 4 : st <= 7 ? 7 : ln ? 0 : st <= 12 ? 12 : st <= 16 ? 16 : st <= 25 ? 25 : 0;
+  if (p.ST == 0) return false;
+  // half tiles where each SM still gets one at most (the norm's products are the wide ones)
+  p.F = !ln && (N + 7) / 8 <= FW_SMS ? 8 : 16;
+  const int tiles = (N + p.F - 1) / p.F;
+  p.blocks = tiles < FW_SMS ? tiles : FW_SMS;
+  const int most = (tiles + p.blocks - 1) / p.blocks;      // tiles of a block
+  const size_t tile = (size_t)p.F * few_pitch(K) * sizeof(bf16);
+  auto fixed = [&](int gt, int s) {
+    return (size_t)(s > 1 ? 2 : 1) * FW_WARPS * gt * FW_ROWS * FW_RED_PITCH * sizeof(float) + (ln ? (size_t)2 * K * sizeof(float) : 0);
+  };
+  // all of a block's tiles as one group in flight, if they are few; else groups of two or one, as many as fit
+  if (most <= (p.ST <= 7 ? 3 : 1) && most * tile + fixed(most, 1) <= FW_SMEM_LIMIT) {
+    p.GT = most;
+    p.stages = 1;
+  } else {
+    p.GT = p.ST <= 7 && 6 * tile + fixed(2, 3) <= FW_SMEM_LIMIT ? 2 : 1;
+    const int groups = (most + p.GT - 1) / p.GT;
+    p.stages = (int)((FW_SMEM_LIMIT - fixed(p.GT, 2)) / (p.GT * tile));
+    if (p.stages > groups) p.stages = groups;
+    if (p.stages > FW_MAX_BARS) p.stages = FW_MAX_BARS;
+    if (p.stages < 2) return false;        // (it would wait for every load)
+  }
+  p.smem = p.stages * p.GT * tile + fixed(p.GT, p.stages);
+  return true;
+}
+
+template <int F, int GT, int ST, bool LN>
+static int launch_few(const FewParams& prm, const FewPlan& p, cudaStream_t stream) {
+  static const cudaError_t attr = cudaFuncSetAttribute(linear_few_kernel<F, GT, ST, LN>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FW_SMEM_LIMIT);
+  if (attr != cudaSuccess) return (int)attr;
+  cudaError_t e = launch_pdl(linear_few_kernel<F, GT, ST, LN>, dim3(p.blocks), dim3(FW_WARPS * 32), p.smem, stream, prm);
+  if (e != cudaSuccess) return (int)e;
+  NIB_LAUNCH_CHECK();
+}
+
+template <int F, int GT, bool LN>
+static int launch_few_st(const FewParams& prm, const FewPlan& p, cudaStream_t stream) {
+  switch (p.ST) {
+    case 3: return launch_few<F, GT, 3, LN>(prm, p, stream);
+    case 4: return launch_few<F, GT, 4, LN>(prm, p, stream);
+    case 7: return launch_few<F, GT, 7, LN>(prm, p, stream);
+  }
+  if constexpr (!LN && GT == 1) {
+    switch (p.ST) {
+      case 12: return launch_few<F, GT, 12, LN>(prm, p, stream);
+      case 16: return launch_few<F, GT, 16, LN>(prm, p, stream);
+      case 25: return launch_few<F, GT, 25, LN>(prm, p, stream);
+    }
+  }
+  return NIB_ERR_UNSUPPORTED_SIZE;
+}
+
+}  // namespace nib
+
+using namespace nib;
+
+// The product for steps of at most 8 rows (bfloat16 weights and activations; out bfloat16 or float32), with the options
+// of nib_linear_skinny.  NIB_ERR_UNSUPPORTED_SIZE where a size or an alignment is not taken.
+extern "C" int nib_linear_few(int out_dtype, const void* a, int lda, const void* w, int ldw, const float* bias, void* out,
+                              int ldo, int M, int N, int K, int act, int residual, const float* ln_x, int ln_ldx,
+                              const float* ln_gamma, const float* ln_beta, float ln_eps, const int* ln_rows, void* cache,
+                              const int* block_table, int max_blocks, const int* row_entry, const int* positions, int q_dim,
+                              int n_kv_head, int head_dim, int page_size, int n_pages, int* status, cudaStream_t stream) {
+  if (N <= 0 || M <= 0) return 0;
+  const bool ln = ln_x != nullptr;
+  FewPlan p;
+  if (!few_plan(M, N, K, ln, p) || (ldw & 7) || ((uintptr_t)w & 15)) return NIB_ERR_UNSUPPORTED_SIZE;
+  if (!ln && a == nullptr) return NIB_ERR_BAD_ARGUMENT;
+  if (residual && out_dtype != DT_F32) return NIB_ERR_BAD_ARGUMENT;
+  if (cache != nullptr && (out_dtype != DT_BF16 || residual || N != q_dim + 2 * n_kv_head * head_dim)) return NIB_ERR_BAD_ARGUMENT;
+  if (!ln && ((lda & 7) || ((uintptr_t)a & 15))) return NIB_ERR_UNSUPPORTED_SIZE;
+  if (ln && ((ln_ldx & 3) || ((uintptr_t)ln_x & 15) || ((uintptr_t)ln_gamma & 15) || ((uintptr_t)ln_beta & 15)))
+    return NIB_ERR_UNSUPPORTED_SIZE;
+  FewParams prm;
+  prm.a = (const bf16*)a; prm.lda = lda;
+  prm.ln_x = ln_x; prm.ln_ldx = ln_ldx; prm.ln_gamma = ln_gamma; prm.ln_beta = ln_beta; prm.ln_rows = ln_rows; prm.ln_eps = ln_eps;
+  prm.w = (const bf16*)w; prm.ldw = ldw; prm.bias = bias; prm.out = out; prm.ldo = ldo;
+  prm.out_f32 = out_dtype == DT_F32; prm.residual = residual; prm.act = act;
+  prm.M = M; prm.N = N; prm.K = K; prm.stages = p.stages;
+  const int tiles = (N + p.F - 1) / p.F;
+  prm.per_block = tiles / p.blocks; prm.wide = tiles % p.blocks;
+  prm.inv_k = (float)(1.0 / K);
+  prm.kv_cache = (bf16*)cache; prm.kv_block_table = block_table; prm.kv_row_entry = row_entry; prm.kv_positions = positions;
+  prm.kv_max_blocks = max_blocks; prm.kv_q_dim = q_dim; prm.kv_heads = n_kv_head; prm.kv_head_dim = head_dim;
+  prm.kv_page_size = page_size; prm.kv_n_pages = n_pages;
+  prm.status = status;
+  if (p.F == 16) {
+    switch (p.GT) {
+      case 1: return ln ? launch_few_st<16, 1, true>(prm, p, stream) : launch_few_st<16, 1, false>(prm, p, stream);
+      case 2: return ln ? launch_few_st<16, 2, true>(prm, p, stream) : launch_few_st<16, 2, false>(prm, p, stream);
+      default: return ln ? launch_few_st<16, 3, true>(prm, p, stream) : launch_few_st<16, 3, false>(prm, p, stream);
+    }
+  }
+  return launch_few_st<8, 1, false>(prm, p, stream);
+}

@@ -57,6 +57,9 @@ _SIGNATURES = {
     "nib_linear_skinny": [_c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int,
                           _c_int, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_float, _c_ptr, _c_ptr, _c_ptr,
                           _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr],
+    "nib_linear_few": [_c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
+                       _c_ptr, _c_int, _c_ptr, _c_ptr, _c_float, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int,
+                       _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr],
     "nib_attention_prefill_tc_supported": [_c_int, _c_int],
     "nib_attention_prefill_tc": [_c_ptr, _c_int, _c_int, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr,
                                  _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_float, _c_int,
@@ -564,6 +567,27 @@ def linear_skinny(a, norm, w, bias, out, M, act=ACT_NONE, residual=False, kv=Non
     return True
 
 
+FEW_MAX_ROWS = 8
+
+
+def linear_few(a, norm, w, bias, out, M, act=ACT_NONE, residual=False, kv=None) -> bool:
+    """The kernel for steps of at most 8 rows (bfloat16): one block an SM, its weights by the copy engine into shared
+    memory, the rows from memory to the MMAs' registers.  Options as for ``linear_skinny``; False where it does not apply."""
+    if M > FEW_MAX_ROWS or not _small_inputs_ok(a, norm, w, out):
+        return False
+    N, K = w.shape
+    ln_args, kv_args = _option_args(norm, kv)
+    if tracing():
+        _note_linear(a, norm, w, bias, out, M, residual)
+    code = library().nib_linear_few(_dt(out), _ptr(a), a.stride(0) if a is not None else 0, _ptr(w), w.stride(0),
+                                    _ptr(bias), _ptr(out), out.stride(0), M, N, K, act, int(residual), *ln_args,
+                                    *kv_args, _ptr(status_word()), _stream())
+    if code == -2:   # alignment or size not taken
+        return False
+    _check(code, "linear_few")
+    return True
+
+
 def linear_small_tc(a, norm, w, bias, out, M, act=ACT_NONE, residual=False, kv=None, split=True) -> bool:
     """The tensor-core kernel for steps of at most 128 rows with its options: ``norm`` folds the
     LayerNorm before the product into the kernel, ``kv`` sends keys and values straight to the
@@ -614,6 +638,9 @@ def _linear_small(a, norm, w, bias, out, M, act, residual, kv=None) -> bool:
     K through scratch, costs more round trips than it saves at these sizes, so that kernel is given
     normed rows and is not split here."""
     N, K = w.shape
+    # (up to 8 rows: measured ahead of the kernel for up to 128 rows at every product of widths 768, 1024 and 1600, see there)
+    if M <= FEW_MAX_ROWS and linear_few(a, norm, w, bias, out, M, act, residual, kv):
+        return True
     mma = skinny_pays(M, N, K)
     if mma:
         # (rows wider than SKINNY_LN_REGISTER_WIDTH are normalised through a buffer per warp in shared memory, which

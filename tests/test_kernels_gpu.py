@@ -806,6 +806,68 @@ def test_few_row_product_with_k_split_over_a_cluster(M, N, K, split):
     assert int(o.status_word().item()) == 0
 
 
+# tiles of 8 and of 16 features on 148 blocks: one tile, a ragged one, one more than the blocks, groups of two and three,
+# a ring of several; steps of K: one piece, a ragged step, the edges between the kernels' numbers of steps
+FEW_SHAPES = [(1, 7, 8, False), (8, 1184, 768, False), (3, 1185, 776, False), (8, 16, 24, True), (1, 2369, 768, True),
+              (8, 4737, 1024, True), (5, 7105, 1032, True), (2, 7200, 1792, True), (8, 9001, 256, False), (8, 768, 3072, False),
+              (7, 1000, 4096, False), (4, 1600, 6400, False), (8, 17, 1600, False)]
+
+
+@pytest.mark.parametrize("M, N, K, ln", FEW_SHAPES)
+def test_product_of_at_most_eight_rows(M, N, K, ln):
+    """The kernel for 1 to 8 rows against 64 bits: its epilogues, a norm with and without shift, rows by a list, what lies
+    beside the result untouched.  Products of bfloat16 are exact in 32 bits, so a 32-bit output is off by the additions'
+    rounding at most; a normalised row may round the other way at a tie, half a unit of bfloat16's last place (2^-8) a value."""
+    o = ops()
+    from nanoinfer_b200.parts.base import Workspace
+    g = gen(M + N + K)
+    a = torch.randn(M + 2, K, generator=g).to(torch.bfloat16)
+    w, b = (torch.randn(N, K, generator=g) * 0.05).to(torch.bfloat16), torch.randn(N, generator=g)
+    wd, bd, ad = w.to(DEV), b.to(DEV), a.to(DEV)
+    norms = [None]
+    if ln:
+        x = torch.randn(M + 2, K, generator=g) * 1.5 - 0.3
+        rows = torch.randperm(M + 2, generator=g)[:M].to(torch.int32)
+        gamma, beta = 1 + 0.1 * torch.randn(K, generator=g), 0.1 * torch.randn(K, generator=g)
+        ws = Workspace(torch.device(DEV))
+        norms = [o.NormInput(x.to(DEV), gamma.to(DEV), be, 1e-5, ws, torch.bfloat16, rows=rows.to(DEV)) for be in (beta.to(DEV), None)]
+    for norm in norms:
+        if norm is None:
+            xn = a[:M].double()
+        elif norm.beta is not None:
+            xn = P.layernorm(x.double(), gamma.double(), beta.double(), 1e-5)[rows.long()]
+        else:
+            xd = x.double()[rows.long()]
+            xn = xd / torch.sqrt((xd * xd).mean(1, keepdim=True) + 1e-5) * gamma.double()
+        xr = xn.to(torch.bfloat16).double()
+        y = xr @ w.double().T + b.double()
+        size = xr.abs() @ w.double().abs().T
+        bound = (K + 16) * 2.0 ** -24 * (size + b.double().abs()) + (2.0 ** -8 * size if norm is not None else 0) + 1e-6
+        inp = None if norm is not None else ad
+        pitch = (N + 15) // 16 * 16
+        buf = torch.full((M + 1, pitch), -7.0, device=DEV)
+        assert o.linear_few(inp, norm, wd, bd, buf[:, :N], M)
+        got = buf.cpu().double()
+        assert ((got[:M, :N] - y).abs() <= bound).all()
+        assert (got[:M, N:] == -7.0).all() and (got[M:] == -7.0).all()
+        res = torch.randn(M, N, generator=g)
+        rd = res.to(DEV)
+        assert o.linear_few(inp, norm, wd, None, rd, M, residual=True)
+        assert ((rd.cpu().double() - (y - b.double() + res.double())).abs() <= bound + 2.0 ** -23 * res.abs()).all()
+        out = torch.full((M + 1, N), 3.0, dtype=torch.bfloat16, device=DEV)
+        assert o.linear_few(inp, norm, wd, bd, out, M, act=o.ACT_CODES["tanh"])
+        ref = P.gelu_tanh(y)
+        # (the hardware's tanh: 2^-10.987 relative; the slope of the function is below 1.13)
+        assert ((out.cpu().double()[:M] - ref).abs() <= 1.13 * bound + 2.0 ** -8 * ref.abs() + 2.0 ** -10.9 * y.abs()).all()
+        assert (out.cpu()[M:] == 3.0).all()
+        if M > 1:     # a row's result does not depend on the rows beside it
+            alone = torch.zeros(1, N, device=DEV)
+            one = None if norm is None else o.NormInput(norm.x, norm.gamma, norm.beta, 1e-5, ws, torch.bfloat16, rows=norm.rows[M - 1:].contiguous())
+            assert o.linear_few(None if norm is not None else ad[M - 1:], one, wd, bd, alone, 1)
+            assert torch.equal(alone[0], buf[M - 1, :N])
+    assert int(o.status_word().item()) == 0
+
+
 PAIR_SHAPES = [(256, 256, 64), (2048, 2304, 768), (2000, 3072, 768), (513, 1000, 264), (1024, 768, 3072), (300, 200, 72)]
 
 
