@@ -56,7 +56,6 @@ struct FewParams {
   int M, N, K;
   int stages;           // groups of tiles in flight
   int per_block, wide;  // tiles a block, and how many blocks have one more
-  float inv_k;          // 1 / K
   bf16* kv_cache;       // optional: features from kv_q_dim on go to the paged cache
   const int* kv_block_table;
   const int* kv_row_entry;
@@ -113,14 +112,6 @@ __device__ __forceinline__ uint32_t pack2x(uint64_t v) {
   split2(v, lo, hi);
   return few_pack(lo, hi);
 }
-// 1 / sqrt(v) for v > 0: the hardware's estimate and one Newton step (a division and a root by the library are calls of
-// 60 and 140 cycles, more where a lane's value is zero, in the middle of a chain of about 3,000)
-__device__ __forceinline__ float few_rsqrt(float v) {
-  const float y = rsqrtf(v);
-  const float z = fmaf(0.5f * y, fmaf(-v * y, y, 1.0f), y);
-  return v < 3.0e38f ? z : y;      // (an overflowed variance: 0, as 1 / sqrt(inf))
-}
-
 // GT: tiles of a group (their sums are added up behind one barrier); ST: 32-wide steps of K a warp has (K <= 256 * ST);
 // warp w takes the steps w, w + 8, ...
 template <int F, int GT, int ST, bool LN>
@@ -220,13 +211,14 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 2) linear_few_kernel(const __gr
   const bool row_here = fr < M;
   const float* xrow = nullptr;
   if (LN && row_here) xrow = prm.ln_x + (size_t)(prm.ln_rows ? prm.ln_rows[fr] : fr) * prm.ln_ldx;
-  float n_vals = 0.0f, inv_n = 0.0f;              // values of a row that this warp sums
+  float n_vals = 0.0f, inv_n = 0.0f, inv_k = 0.0f;              // values of a row that this warp sums
   if (LN) {
     int n = 0;
 #pragma unroll
     for (int s = 0; s < ST; ++s) n += 8 * max(0, min(4, n_chunks - 4 * (warp + s * FW_WARPS)));
     n_vals = (float)n;
-    inv_n = n > 0 ? 1.0f / n_vals : 0.0f;
+    inv_n = n > 0 ? reciprocal_ahead(n) : 0.0f;
+    inv_k = reciprocal_ahead(K);
   }
   __syncthreads();             // the barriers are initialised
   pdl_wait();
@@ -286,10 +278,10 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 2) linear_few_kernel(const __gr
     float4 st[FW_WARPS];
 #pragma unroll
     for (int w = 0; w < FW_WARPS; ++w) { st[w] = stats[w][fr]; total += st[w].x; }
-    const float mean = shifted ? total * prm.inv_k : 0.0f;
+    const float mean = shifted ? total * inv_k : 0.0f;
 #pragma unroll
     for (int w = 0; w < FW_WARPS; ++w) { const float d = st[w].z - mean; squares += st[w].y + st[w].w * d * d; }
-    const float rstd = few_rsqrt(squares * prm.inv_k + prm.ln_eps);
+    const float rstd = inv_sqrt(squares * inv_k + prm.ln_eps);
     const uint64_t mm = two(-mean, -mean), rr = two(rstd, rstd);
 #pragma unroll
     for (int s = 0; s < ST; ++s) {
@@ -504,7 +496,6 @@ extern "C" int nib_linear_few(int out_dtype, const void* a, int lda, const void*
   prm.M = M; prm.N = N; prm.K = K; prm.stages = p.stages;
   const int tiles = (N + p.F - 1) / p.F;
   prm.per_block = tiles / p.blocks; prm.wide = tiles % p.blocks;
-  prm.inv_k = (float)(1.0 / K);
   prm.kv_cache = (bf16*)cache; prm.kv_block_table = block_table; prm.kv_row_entry = row_entry; prm.kv_positions = positions;
   prm.kv_max_blocks = max_blocks; prm.kv_q_dim = q_dim; prm.kv_heads = n_kv_head; prm.kv_head_dim = head_dim;
   prm.kv_page_size = page_size; prm.kv_n_pages = n_pages;

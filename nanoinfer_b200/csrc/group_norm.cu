@@ -73,6 +73,7 @@ group_norm_vec_kernel(Src src, const float* __restrict__ w, OutT* out, int n_row
     for (int i = 0; i < NV; ++i)
       if (lane + 32 * i < n4) ww[i] = gn_load4(w + c0 + 4 * (lane + 32 * i));
   }
+  const float inv_n = reciprocal_ahead(gs);
   pdl_wait();
   if (r >= n_rows) return;
   auto* p = src.row(r, C) + c0;
@@ -100,7 +101,7 @@ group_norm_vec_kernel(Src src, const float* __restrict__ w, OutT* out, int n_row
     }
   }
   if (out == nullptr) return;
-  const float rstd = 1.0f / sqrtf(warp_sum(q) / (float)gs + eps);
+  const float rstd = inv_sqrt(warp_sum(q) * inv_n + eps);
   OutT* o = out + (size_t)r * C + c0;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
@@ -127,6 +128,7 @@ group_norm_row_kernel(Src src, const float* __restrict__ w, OutT* out, int n_row
       if (k < n4) ww[i] = gn_load4(w + 4 * k);
     }
   }
+  const float inv_n = reciprocal_ahead(C);
   pdl_wait();
   auto* p = src.row(r, C);
   float4 v[NV];
@@ -153,7 +155,7 @@ group_norm_row_kernel(Src src, const float* __restrict__ w, OutT* out, int n_row
     }
   }
   if (out == nullptr) return;
-  const float rstd = 1.0f / sqrtf(block_sum(q, sums) / (float)C + eps);
+  const float rstd = inv_sqrt(block_sum(q, sums) * inv_n + eps);
   OutT* o = out + (size_t)r * C;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
@@ -171,6 +173,7 @@ group_norm_any_kernel(Src src, const float* __restrict__ w, OutT* out, int n_row
   const int unit = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int r = unit / groups, g = unit % groups;
   const int gs = C / groups, c0 = g * gs;
+  const float inv_n = reciprocal_ahead(gs);
   pdl_wait();
   if (r >= n_rows) return;
   auto* p = src.row(r, C) + c0;
@@ -187,7 +190,7 @@ group_norm_any_kernel(Src src, const float* __restrict__ w, OutT* out, int n_row
     q += v * v;
   }
   if (out == nullptr) return;
-  const float rstd = 1.0f / sqrtf(warp_sum(q) / (float)gs + eps);
+  const float rstd = inv_sqrt(warp_sum(q) * inv_n + eps);
   OutT* o = out + (size_t)r * C + c0;
   for (int c = lane; c < gs; c += 32) {      // (a lane reads again what it read, or wrote, itself)
     float v = to_float(p[c]);

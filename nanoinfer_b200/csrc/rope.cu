@@ -112,6 +112,7 @@ norm_rope_append_kernel(const float* proj, int ld, int q_off, int k_off, int v_o
       dst = cache + kv_offset(page, is_k ? 0 : 1, h, pos % page_size, n_kv_head, page_size, hd);
     }
   }
+  const float inv_dim = reciprocal_ahead(is_q || is_k ? dim : vdim);
   pdl_wait();
   if (dst == nullptr) return;
   const int width = is_q || is_k ? dim : vdim;
@@ -126,7 +127,7 @@ norm_rope_append_kernel(const float* proj, int ld, int q_off, int k_off, int v_o
     ss += x[i].x * x[i].x + x[i].y * x[i].y;
   }
   float r = 1.0f;
-  if (w != nullptr) r = 1.0f / sqrtf(warp_sum(ss) / (float)width + eps);
+  if (w != nullptr) r = inv_sqrt(warp_sum(ss) * inv_dim + eps);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int c = 2 * (lane + 32 * i);
@@ -420,6 +421,7 @@ norm_rope_maps_append_kernel(const float* proj, int ld, int q_off, int k_off, in
       page = -1;
     }
   }
+  const float inv_dim = reciprocal_ahead(dim);
   pdl_wait();
   for (int u = blockIdx.x * n_warps + warp; u < nq + nk + n_kv_head; u += gridDim.x * n_warps) {
     const bool is_q = u < nq, is_k = !is_q && u < nq + nk;
@@ -446,7 +448,7 @@ norm_rope_maps_append_kernel(const float* proj, int ld, int q_off, int k_off, in
       x[k] = c < dim ? src[c] : 0.0f;
       ss += x[k] * x[k];
     }
-    const float r = w != nullptr ? 1.0f / sqrtf(warp_sum(ss) / (float)dim + eps) : 1.0f;
+    const float r = w != nullptr ? inv_sqrt(warp_sum(ss) * inv_dim + eps) : 1.0f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int c = lane + 32 * k;
