@@ -1,4 +1,5 @@
-// out = act(a . w^T + bias) for steps of one to eight rows, in bfloat16: a decode step of a few requests.
+// out = act(a . w^T + bias) for steps of one to eight rows, in bfloat16: a decode step of a few requests.  (The entry point
+// takes steps of up to 128 rows and hands those of more than eight to gemm_few_rows.cu.)
 //
 // Such a product is a stream of weights with a handful of multiply-adds each, one of a hundred dependent launches of a
 // step, and what counts is the chain from the end of the kernel ahead to its own last store.  (A launch boundary under
@@ -27,91 +28,12 @@
 // What is left at 8 rows of small: 0.5 us launch, 0.3 for the stores to be visible, about 0.4 until the rows are here,
 // 0.45 statistics and normalisation, 0.25 MMAs, 0.3 sums across warps and epilogue; at XL's sizes the weights' way into
 // shared memory (104 to 205 KB an SM).
-#include "api.h"
-#include "tcgen05.cuh"
+#include "gemm_few.cuh"
 
 namespace nib {
 
-constexpr int FW_WARPS = 8;
-constexpr int FW_ROWS = 8;            // rows of a step, at most
-constexpr int FW_SMS = 148;
-constexpr int FW_MAX_BARS = 16;       // groups of tiles in flight, at most
-constexpr int FW_RED_PITCH = 20;      // floats between the rows of a tile's partial sums (16 features): no bank conflicts
-constexpr size_t FW_SMEM_LIMIT = 220 * 1024;
+constexpr int FW_ROWS = 8;
 
-struct FewParams {
-  const bf16* a;        // [M, K] activations (LN: unused)
-  int lda;
-  const float* ln_x;    // LN: the residual stream, normalised here
-  int ln_ldx;
-  const float* ln_gamma;
-  const float* ln_beta;   // null: an RMS norm (nothing is taken off, nothing added)
-  const int* ln_rows;
-  float ln_eps;
-  const bf16* w;        // [N, K]
-  int ldw;
-  const float* bias;
-  void* out;
-  int ldo, out_f32, residual, act;
-  int M, N, K;
-  int stages;           // groups of tiles in flight
-  int per_block, wide;  // tiles a block, and how many blocks have one more
-  bf16* kv_cache;       // optional: features from kv_q_dim on go to the paged cache
-  const int* kv_block_table;
-  const int* kv_row_entry;
-  const int* kv_positions;
-  int kv_max_blocks, kv_q_dim, kv_heads, kv_head_dim, kv_page_size, kv_n_pages;
-  int* status;
-};
-
-__device__ __forceinline__ void few_mma(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t few_pack(float lo, float hi) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
-// one row of weights, `bytes` (a multiple of 16), both addresses on 16 bytes
-__device__ __forceinline__ void few_bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
-// elements between the weight rows of a tile: pieces of 8 rows x 4 lanes hit distinct banks
-__host__ __device__ inline int few_pitch(int K) { return K + ((32 - K % 64) + 64) % 64; }
-
-// two 32-bit values in one register pair
-__device__ __forceinline__ uint64_t two(float lo, float hi) {
-  uint64_t v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-  return v;
-}
-__device__ __forceinline__ void split2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint32_t pack2x(uint64_t v) {
-  float lo, hi;
-  split2(v, lo, hi);
-  return few_pack(lo, hi);
-}
 // GT: tiles of a group (their sums are added up behind one barrier); ST: 32-wide steps of K a warp has (K <= 256 * ST);
 // warp w takes the steps w, w + 8, ...
 template <int F, int GT, int ST, bool LN>
@@ -407,30 +329,24 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 2) linear_few_kernel(const __gr
   }
 }
 
-// How a product is cut: F features a tile, GT tiles a group, ST steps a warp, stages of groups in flight.
-struct FewPlan { int F, GT, ST, stages, blocks; size_t smem; };
-
-static bool few_plan(int M, int N, int K, bool ln, FewPlan& p) {
-  if (M < 1 || M > FW_ROWS || N < 1 || K < 8 || (K & 7)) return false;
-  const int st = (K + 255) / 256;
-  p.ST = st <= 3 ? 3 : st <= 4 ? 4 : st <= 7 ? 7 : ln ? 0 : st <= 12 ? 12 : st <= 16 ? 16 : st <= 25 ? 25 : 0;
-  if (p.ST == 0) return false;
-  // half tiles where each SM still gets one at most (the norm's products are the wide ones)
-  p.F = !ln && (N + 7) / 8 <= FW_SMS ? 8 : 16;
-  const int tiles = (N + p.F - 1) / p.F;
-  p.blocks = tiles < FW_SMS ? tiles : FW_SMS;
+static bool few_cut(int M, int N, int K, bool ln, int F, FewPlan& p) {
+  p.F = F;
+  const int places = FW_SMS / p.row_blocks;                // blocks of a row block
+  const int tiles = (N + F - 1) / F;
+  p.blocks = tiles < places ? tiles : places;
   const int most = (tiles + p.blocks - 1) / p.blocks;      // tiles of a block
-  const size_t tile = (size_t)p.F * few_pitch(K) * sizeof(bf16);
+  const size_t tile = (size_t)F * few_pitch(K) * sizeof(bf16);
   auto fixed = [&](int gt, int s) {
-    return (size_t)(s > 1 ? 2 : 1) * FW_WARPS * gt * FW_ROWS * FW_RED_PITCH * sizeof(float) + (ln ? (size_t)2 * K * sizeof(float) : 0);
+    return (size_t)(s > 1 ? 2 : 1) * FW_WARPS * gt * 8 * p.NT * FW_RED_PITCH * sizeof(float) + (ln ? (size_t)2 * K * sizeof(float) : 0);
   };
   // all of a block's tiles as one group in flight, if they are few; else groups of two or one, as many as fit
-  if (most <= (p.ST <= 7 ? 3 : 1) && most * tile + fixed(most, 1) <= FW_SMEM_LIMIT) {
+  if (most <= (F == 16 && p.ST <= 7 ? 3 : 1) && most * tile + fixed(most, 1) <= FW_SMEM_LIMIT) {
     p.GT = most;
     p.stages = 1;
   } else {
-    p.GT = p.ST <= 7 && 6 * tile + fixed(2, 3) <= FW_SMEM_LIMIT ? 2 : 1;
+    p.GT = F == 16 && p.ST <= 7 && 4 * tile + fixed(2, 2) <= FW_SMEM_LIMIT ? 2 : 1;
     const int groups = (most + p.GT - 1) / p.GT;
+    if (fixed(p.GT, 2) >= FW_SMEM_LIMIT) return false;
     p.stages = (int)((FW_SMEM_LIMIT - fixed(p.GT, 2)) / (p.GT * tile));
     if (p.stages > groups) p.stages = groups;
     if (p.stages > FW_MAX_BARS) p.stages = FW_MAX_BARS;
@@ -440,12 +356,26 @@ static bool few_plan(int M, int N, int K, bool ln, FewPlan& p) {
   return true;
 }
 
+static bool few_plan(int M, int N, int K, bool ln, FewPlan& p) {
+  if (M < 1 || M > FW_MAX_ROWS || N < 1 || K < 8 || (K & 7)) return false;
+  p.NT = M <= 8 ? 1 : 2;
+  p.row_blocks = (M + 8 * p.NT - 1) / (8 * p.NT);
+  const int st = (K + 255) / 256;
+  p.ST = st <= 3 ? 3 : st <= 4 ? 4 : st <= 7 ? 7 : ln ? 0 : st <= 12 ? 12 : st <= 16 ? 16 : st <= 25 ? 25 : 0;
+  if (p.ST == 0) return false;
+  if (ln) return few_cut(M, N, K, ln, 16, p);
+  // half tiles where each SM still gets one at most (the norm's products are the wide ones), or where whole ones do not fit
+  const bool narrow = (N + 7) / 8 <= FW_SMS / p.row_blocks;
+  return few_cut(M, N, K, ln, narrow ? 8 : 16, p) || (!narrow && few_cut(M, N, K, ln, 8, p));
+}
+
 template <int F, int GT, int ST, bool LN>
 static int launch_few(const FewParams& prm, const FewPlan& p, cudaStream_t stream) {
   static const cudaError_t attr = cudaFuncSetAttribute(linear_few_kernel<F, GT, ST, LN>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FW_SMEM_LIMIT);
   if (attr != cudaSuccess) return (int)attr;
-  cudaError_t e = launch_pdl(linear_few_kernel<F, GT, ST, LN>, dim3(p.blocks), dim3(FW_WARPS * 32), p.smem, stream, prm);
+  cudaError_t e = launch_pdl(linear_few_kernel<F, GT, ST, LN>, dim3(p.blocks), dim3(FW_WARPS * 32), p.smem,
+                             stream, prm);
   if (e != cudaSuccess) return (int)e;
   NIB_LAUNCH_CHECK();
 }
@@ -465,6 +395,15 @@ static int launch_few_st(const FewParams& prm, const FewPlan& p, cudaStream_t st
     }
   }
   return NIB_ERR_UNSUPPORTED_SIZE;
+}
+
+static int launch_few_one(const FewParams& prm, const FewPlan& p, bool ln, cudaStream_t stream) {
+  if (p.F == 8) return launch_few_st<8, 1, false>(prm, p, stream);
+  switch (p.GT) {
+    case 1: return ln ? launch_few_st<16, 1, true>(prm, p, stream) : launch_few_st<16, 1, false>(prm, p, stream);
+    case 2: return ln ? launch_few_st<16, 2, true>(prm, p, stream) : launch_few_st<16, 2, false>(prm, p, stream);
+    default: return ln ? launch_few_st<16, 3, true>(prm, p, stream) : launch_few_st<16, 3, false>(prm, p, stream);
+  }
 }
 
 }  // namespace nib
@@ -500,12 +439,5 @@ extern "C" int nib_linear_few(int out_dtype, const void* a, int lda, const void*
   prm.kv_max_blocks = max_blocks; prm.kv_q_dim = q_dim; prm.kv_heads = n_kv_head; prm.kv_head_dim = head_dim;
   prm.kv_page_size = page_size; prm.kv_n_pages = n_pages;
   prm.status = status;
-  if (p.F == 16) {
-    switch (p.GT) {
-      case 1: return ln ? launch_few_st<16, 1, true>(prm, p, stream) : launch_few_st<16, 1, false>(prm, p, stream);
-      case 2: return ln ? launch_few_st<16, 2, true>(prm, p, stream) : launch_few_st<16, 2, false>(prm, p, stream);
-      default: return ln ? launch_few_st<16, 3, true>(prm, p, stream) : launch_few_st<16, 3, false>(prm, p, stream);
-    }
-  }
-  return launch_few_st<8, 1, false>(prm, p, stream);
+  return p.NT == 1 ? launch_few_one(prm, p, ln, stream) : launch_few_rows(prm, p, ln, stream);
 }

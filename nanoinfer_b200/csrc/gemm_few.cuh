@@ -1,0 +1,92 @@
+// What the products of few rows share (gemm_few.cu: one to eight rows; gemm_few_rows.cu: blocks of sixteen).
+#pragma once
+#include "api.h"
+#include "tcgen05.cuh"
+
+namespace nib {
+
+constexpr int FW_WARPS = 8;
+constexpr int FW_MAX_ROWS = 128;      // rows of a step, at most: row blocks of sixteen beyond eight
+constexpr int FW_SMS = 148;
+constexpr int FW_MAX_BARS = 16;       // groups of tiles in flight, at most
+constexpr int FW_RED_PITCH = 20;      // floats between the rows of a tile's partial sums (16 features): no bank conflicts
+constexpr size_t FW_SMEM_LIMIT = 220 * 1024;
+
+struct FewParams {
+  const bf16* a;        // [M, K] activations (LN: unused)
+  int lda;
+  const float* ln_x;    // LN: the residual stream, normalised here
+  int ln_ldx;
+  const float* ln_gamma;
+  const float* ln_beta;   // null: an RMS norm (nothing is taken off, nothing added)
+  const int* ln_rows;
+  float ln_eps;
+  const bf16* w;        // [N, K]
+  int ldw;
+  const float* bias;
+  void* out;
+  int ldo, out_f32, residual, act;
+  int M, N, K;
+  int stages;           // groups of tiles in flight
+  int per_block, wide;  // tiles a block, and how many blocks have one more
+  bf16* kv_cache;       // optional: features from kv_q_dim on go to the paged cache
+  const int* kv_block_table;
+  const int* kv_row_entry;
+  const int* kv_positions;
+  int kv_max_blocks, kv_q_dim, kv_heads, kv_head_dim, kv_page_size, kv_n_pages;
+  int* status;
+};
+
+__device__ __forceinline__ void few_mma(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t few_pack(float lo, float hi) {
+  __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
+// one row of weights, `bytes` (a multiple of 16), both addresses on 16 bytes
+__device__ __forceinline__ void few_bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+// elements between the weight rows of a tile: pieces of 8 rows x 4 lanes hit distinct banks
+__host__ __device__ inline int few_pitch(int K) { return K + ((32 - K % 64) + 64) % 64; }
+
+// two 32-bit values in one register pair
+__device__ __forceinline__ uint64_t two(float lo, float hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ void split2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint32_t pack2x(uint64_t v) {
+  float lo, hi;
+  split2(v, lo, hi);
+  return few_pack(lo, hi);
+}
+// How a product is cut: F features a tile, GT tiles a group, ST steps a warp, blocks of 8 * NT rows, stages of groups in flight.
+struct FewPlan { int F, GT, ST, NT, stages, blocks, row_blocks; size_t smem; };
+int launch_few_rows(const FewParams& prm, const FewPlan& p, bool ln, cudaStream_t stream);   // (NT = 2)
+
+}  // namespace nib

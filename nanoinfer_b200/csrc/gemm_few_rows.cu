@@ -1,0 +1,383 @@
+// The product of gemm_few.cu for steps of 9 to 128 rows: row blocks of sixteen (grid y), each with its share of the SMs, so
+// that a block's chain is as long as in a step of sixteen rows but for the tiles that it walks (the ring of stages).  A lane
+// has two rows, fr and fr + 8: two MMAs a weight where weights are the 16-row operand, one where the rows are.
+// A kernel of its own, for its code and for its registers (one block an SM): with both numbers of rows as one template the
+// kernels of eight rows came out otherwise scheduled and a decode step of GPT-2 small at 8 rows took 286 us instead of 265.
+// Measured (B200, in a graph, weights from memory, us a launch; gemm_skinny.cu or tcgen05 with the norm ahead before, this now):
+//   16 rows, width 768   q/k/v 5.3, 3.8   output 2.8, 2.3   MLP 5.6, 4.3   4.8, 3.9     width 1600  11.7, 7.7  4.8, 3.2  12.5, 8.6  10.4, 8.2
+//   48 rows, width 768         7.0, 5.5          3.2, 2.7       7.3, 6.5   5.5, 4.3     width 1024   8.4, 7.7  3.8, 3.3  10.0, 9.4  6.4, -
+// (bound by what an SM takes in: each row block reads all weights, and each block all its sixteen rows)
+#include "gemm_few.cuh"
+
+namespace nib {
+
+// GT: tiles of a group (their sums are added up behind one barrier); ST: 32-wide steps of K a warp has (K <= 256 * ST);
+// warp w takes the steps w, w + 8, ...
+template <int F, int GT, int ST, bool LN>
+__global__ void __launch_bounds__(FW_WARPS * 32, 1) linear_few_rows_kernel(const __grid_constant__ FewParams prm) {
+  pdl_trigger();
+  constexpr int NT = 2, ROWS = 8 * NT;      // rows of a block, in eights
+  constexpr int R = LN || ST <= 8 ? ST : 8;                // steps of the row that a lane holds at a time
+  constexpr int CH = F == 16 ? (GT == 1 ? 2 : 1) : 4;   // independent chains of MMAs a tile
+  constexpr int TILE_SUMS = ROWS * F;
+  constexpr int OUTS = (GT * TILE_SUMS + FW_WARPS * 32 - 1) / (FW_WARPS * 32);
+  extern __shared__ __align__(128) uint8_t fw_smem[];
+  __shared__ __align__(8) uint64_t bars[FW_MAX_BARS];
+  __shared__ float4 stats[FW_WARPS][ROWS];
+  __shared__ int abort_sh;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31, fr = lane >> 2, kl = lane & 3;
+  const int row0 = blockIdx.y * ROWS;
+  const int M = min(prm.M - row0, ROWS), N = prm.N, K = prm.K, n_chunks = K >> 3;
+  const int pitch = few_pitch(K);
+  // this block's tiles: the first `wide` blocks have one more
+  const int t_begin = blockIdx.x * prm.per_block + min((int)blockIdx.x, prm.wide);
+  const int mine = prm.per_block + ((int)blockIdx.x < prm.wide ? 1 : 0);
+  const int groups = (mine + GT - 1) / GT, S = prm.stages;
+  bf16* ws = reinterpret_cast<bf16*>(fw_smem);             // [stages][GT][F][pitch]
+  float* red = reinterpret_cast<float*>(fw_smem + (size_t)S * GT * F * pitch * sizeof(bf16));
+  constexpr int RED = FW_WARPS * GT * ROWS * FW_RED_PITCH;   // [2][warps][GT][rows][pitch]
+  float* gb = red + (S > 1 ? 2 : 1) * RED;                 // LN: [2][K] scale and shift
+
+  // ---- Before the wait: what the kernel ahead does not write.
+  if (LN) {   // (ahead of the weights: they are needed first)
+    for (int i = threadIdx.x; i < K / 4; i += FW_WARPS * 32) {
+      cp_async16(gb + i * 4, prm.ln_gamma + i * 4, true);
+      cp_async16(gb + K + i * 4, prm.ln_beta != nullptr ? prm.ln_beta + i * 4 : prm.ln_gamma, prm.ln_beta != nullptr);
+    }
+    cp_async_commit();
+  }
+  auto ask = [&](int g, int slot) {      // (the first warp) the weights of group g
+    // (a group's tiles are neighbours: one run of rows here and there)
+    const int f0 = (t_begin + g * GT) * F, rows = min(min(GT, mine - g * GT) * F, N - f0);
+    if (elect_one()) {
+      mbar_expect_tx(&bars[slot], (uint32_t)rows * K * 2);
+      const bf16* src = prm.w + (size_t)f0 * prm.ldw;
+      bf16* dst = ws + (size_t)slot * GT * F * pitch;
+      for (int r = 0; r < rows; ++r) few_bulk_load(dst + (size_t)r * pitch, src + (size_t)r * prm.ldw, (uint32_t)K * 2, &bars[slot]);
+    }
+  };
+  if (warp == 0) {
+    if (elect_one()) {
+      abort_sh = 0;
+      for (int i = 0; i < S; ++i) mbar_init(&bars[i], 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    for (int g = 0; g < S && g < groups; ++g) ask(g, g);
+  }
+  // output q of this thread within a group: tile, row and feature
+  auto place = [&](int q, int& j, int& m, int& nl) {
+    const int o = threadIdx.x + q * FW_WARPS * 32;
+    j = o / TILE_SUMS; m = (o % TILE_SUMS) / F; nl = o % F;
+    return o < GT * TILE_SUMS && m < M;
+  };
+  float bias_r[OUTS], res_r[OUTS];
+  long long kv_at[OUTS];   // where in the cache layer the output goes (-1: to `out`, -2: nowhere, -3: the page is none of the pool's)
+  auto fetch = [&](int g) {   // bias and destination of group g's outputs
+#pragma unroll
+    for (int q = 0; q < OUTS; ++q) {
+      int j, m, nl;
+      const bool ok = place(q, j, m, nl) && g * GT + j < mine;
+      const int n = (t_begin + g * GT + j) * F + nl;
+      bias_r[q] = 0.0f;
+      kv_at[q] = -1;
+      if (ok && n < N) {
+        if (prm.bias != nullptr) bias_r[q] = prm.bias[n];
+        if (prm.kv_cache != nullptr && n >= prm.kv_q_dim) {
+          const int pos = prm.kv_positions[row0 + m], entry = prm.kv_row_entry[row0 + m];
+          const int page = entry < 0 ? 0 : prm.kv_block_table[(size_t)entry * prm.kv_max_blocks + pos / prm.kv_page_size];
+          const int kv_dim = prm.kv_heads * prm.kv_head_dim, rem = n - prm.kv_q_dim, which = rem >= kv_dim ? 1 : 0;
+          const int at = rem - which * kv_dim, head = at / prm.kv_head_dim;
+          kv_at[q] = entry < 0 ? -2
+                     : (page < 0 || page >= prm.kv_n_pages)
+                         ? -3
+                         : (long long)kv_offset(page, which, head, pos % prm.kv_page_size, prm.kv_heads, prm.kv_page_size,
+                                                prm.kv_head_dim) + (at - head * prm.kv_head_dim);
+        }
+      }
+    }
+  };
+  auto fetch_residual = [&](int g) {
+#pragma unroll
+    for (int q = 0; q < OUTS; ++q) {
+      int j, m, nl;
+      const bool ok = place(q, j, m, nl) && g * GT + j < mine;
+      const int n = (t_begin + g * GT + j) * F + nl;
+      res_r[q] = 0.0f;
+      if (ok && prm.residual && n < N) res_r[q] = ((const float*)prm.out)[(size_t)(row0 + m) * prm.ldo + n];
+    }
+  };
+  fetch(0);
+  bool row_here[NT];           // this lane's rows, fr and fr + 8
+  const float* xrow[NT];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    row_here[t] = t * 8 + fr < M;
+    const int r = row0 + t * 8 + fr;
+    xrow[t] = LN && row_here[t] ? prm.ln_x + (size_t)(prm.ln_rows ? prm.ln_rows[r] : r) * prm.ln_ldx : nullptr;
+  }
+  float n_vals = 0.0f, inv_n = 0.0f, inv_k = 0.0f;              // values of a row that this warp sums
+  if (LN) {
+    int n = 0;
+#pragma unroll
+    for (int s = 0; s < ST; ++s) n += 8 * max(0, min(4, n_chunks - 4 * (warp + s * FW_WARPS)));
+    n_vals = (float)n;
+    inv_n = n > 0 ? reciprocal_ahead(n) : 0.0f;
+    inv_k = reciprocal_ahead(K);
+  }
+  __syncthreads();             // the barriers are initialised
+  pdl_wait();
+
+  // ---- the step's rows, in the order of the MMA's operands: of step s, the eight values at (warp + 8 s) * 32 + 8 kl
+  uint4 xb[NT][R];
+  auto load_x = [&](int t, int s) {
+    const int c = (warp + s * FW_WARPS) * 4 + kl;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (row_here[t] && c < n_chunks) v = *reinterpret_cast<const uint4*>(prm.a + (size_t)(row0 + t * 8 + fr) * prm.lda + c * 8);
+    return v;
+  };
+  if (!LN) {
+#pragma unroll
+    for (int s = 0; s < R; ++s)
+#pragma unroll
+      for (int t = 0; t < NT; ++t) xb[t][s] = load_x(t, s);
+  }
+  if constexpr (LN) {
+    uint64_t xf[NT][ST][4];    // pairs of neighbours
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int s = 0; s < ST; ++s) {
+        const int c = (warp + s * FW_WARPS) * 4 + kl;
+        ulonglong2 lo = make_ulonglong2(0, 0), hi = lo;
+        if (row_here[t] && c < n_chunks) {
+          lo = *reinterpret_cast<const ulonglong2*>(xrow[t] + c * 8);
+          hi = *reinterpret_cast<const ulonglong2*>(xrow[t] + c * 8 + 4);
+        }
+        xf[t][s][0] = lo.x; xf[t][s][1] = lo.y; xf[t][s][2] = hi.x; xf[t][s][3] = hi.y;
+      }
+    // this warp's sum and its squared differences from its own mean; then all warps' merged (an RMS norm: mean 0)
+    const bool shifted = prm.ln_beta != nullptr;
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      uint64_t s2 = 0;
+#pragma unroll
+      for (int s = 0; s < ST; ++s) s2 = add2(s2, add2(add2(xf[t][s][0], xf[t][s][1]), add2(xf[t][s][2], xf[t][s][3])));
+      float sum, sum_hi;
+      split2(s2, sum, sum_hi);
+      sum += sum_hi;
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      const float own = shifted ? sum * inv_n : 0.0f;
+      uint64_t q2 = 0;
+#pragma unroll
+      for (int s = 0; s < ST; ++s) {
+        const float c0 = (warp + s * FW_WARPS) * 4 + kl < n_chunks ? -own : 0.0f;   // (zeros past the row)
+        const uint64_t cc = two(c0, c0);
+        const uint64_t d0 = add2(xf[t][s][0], cc), d1 = add2(xf[t][s][1], cc), d2 = add2(xf[t][s][2], cc), d3 = add2(xf[t][s][3], cc);
+        q2 = add2(q2, add2(fma2(d0, d0, mul2(d1, d1)), fma2(d2, d2, mul2(d3, d3))));
+      }
+      float sq, sq_hi;
+      split2(q2, sq, sq_hi);
+      sq += sq_hi;
+      sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+      sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+      if (kl == 0) stats[warp][t * 8 + fr] = make_float4(sum, sq, own, n_vals);
+    }
+    cp_async_wait<0>();        // (the norm's parameters)
+    __syncthreads();
+    uint64_t mm[NT], rr[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      float total = 0.0f, squares = 0.0f;
+      float4 st[FW_WARPS];
+#pragma unroll
+      for (int w = 0; w < FW_WARPS; ++w) { st[w] = stats[w][t * 8 + fr]; total += st[w].x; }
+      const float mean = shifted ? total * inv_k : 0.0f;
+#pragma unroll
+      for (int w = 0; w < FW_WARPS; ++w) { const float d = st[w].z - mean; squares += st[w].y + st[w].w * d * d; }
+      const float rstd = inv_sqrt(squares * inv_k + prm.ln_eps);
+      mm[t] = two(-mean, -mean);
+      rr[t] = two(rstd, rstd);
+    }
+#pragma unroll
+    for (int s = 0; s < ST; ++s) {
+      const int cc = (warp + s * FW_WARPS) * 4 + kl;
+      const int c = cc < n_chunks ? cc : 0;      // (no branch: the steps' chains run side by side)
+      const ulonglong2 g0 = *reinterpret_cast<const ulonglong2*>(gb + c * 8), g1 = *reinterpret_cast<const ulonglong2*>(gb + c * 8 + 4);
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(gb + K + c * 8), b1 = *reinterpret_cast<const ulonglong2*>(gb + K + c * 8 + 4);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        const bool ok = row_here[t] && cc < n_chunks;
+        xb[t][s].x = ok ? pack2x(fma2(mul2(add2(xf[t][s][0], mm[t]), rr[t]), g0.x, b0.x)) : 0u;
+        xb[t][s].y = ok ? pack2x(fma2(mul2(add2(xf[t][s][1], mm[t]), rr[t]), g0.y, b0.y)) : 0u;
+        xb[t][s].z = ok ? pack2x(fma2(mul2(add2(xf[t][s][2], mm[t]), rr[t]), g1.x, b1.x)) : 0u;
+        xb[t][s].w = ok ? pack2x(fma2(mul2(add2(xf[t][s][3], mm[t]), rr[t]), g1.y, b1.y)) : 0u;
+      }
+    }
+  }
+  fetch_residual(0);
+
+  volatile int* abort_flag = &abort_sh;
+  int slot = 0, round = 0;     // g % S, g / S
+#pragma unroll 1
+  for (int g = 0; g < groups; ++g) {
+    if (g > 0) {
+      fetch(g);
+      fetch_residual(g);
+      if (R < ST) {
+#pragma unroll
+        for (int s = 0; s < R; ++s)
+#pragma unroll
+          for (int t = 0; t < NT; ++t) xb[t][s] = load_x(t, s);
+      }
+    }
+    constexpr int AT = F == 16 ? NT : 1;       // accumulators of a tile (F = 8: its MMA has all sixteen rows)
+    float acc[GT][AT][CH][4];
+#pragma unroll
+    for (int j = 0; j < GT; ++j)
+#pragma unroll
+      for (int t = 0; t < AT; ++t)
+#pragma unroll
+        for (int c = 0; c < CH; ++c) acc[j][t][c][0] = acc[j][t][c][1] = acc[j][t][c][2] = acc[j][t][c][3] = 0.0f;
+    const bf16* w0 = ws + ((size_t)slot * GT * F + fr) * pitch;
+    mbar_wait(&bars[slot], round & 1, abort_flag);
+#pragma unroll
+    for (int s = 0; s < ST; ++s) {
+      const int c = (warp + s * FW_WARPS) * 4 + kl;
+      uint4 x[NT];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        x[t] = xb[t][s % R];
+        if (R < ST && s + R < ST) xb[t][s % R] = load_x(t, s + R);
+      }
+#pragma unroll
+      for (int j = 0; j < GT; ++j) {
+        // (past the row, and of a tile that this block does not have: zeros, not what the memory held)
+        uint4 wa = make_uint4(0, 0, 0, 0), wb = wa;
+        if (c < n_chunks && (j == 0 || g * GT + j < mine)) {
+          wa = *reinterpret_cast<const uint4*>(w0 + (size_t)j * F * pitch + c * 8);
+          if (F == 16) wb = *reinterpret_cast<const uint4*>(w0 + ((size_t)j * F + 8) * pitch + c * 8);
+        }
+        if (F == 16) {
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            few_mma(acc[j][t % AT][s % CH], wa.x, wb.x, wa.y, wb.y, x[t].x, x[t].y);
+            few_mma(acc[j][t % AT][s % CH], wa.z, wb.z, wa.w, wb.w, x[t].z, x[t].w);
+          }
+        } else {
+          few_mma(acc[j][0][s % CH], x[0].x, x[1].x, x[0].y, x[1].y, wa.x, wa.y);
+          few_mma(acc[j][0][s % CH], x[0].z, x[1].z, x[0].w, x[1].w, wa.z, wa.w);
+        }
+      }
+    }
+    // ---- the warps' sums meet in shared memory, [row][feature]
+    float* rd = red + (S > 1 ? (g & 1) * RED : 0);
+#pragma unroll
+    for (int j = 0; j < GT; ++j) {
+      float* r0 = rd + (warp * GT + j) * ROWS * FW_RED_PITCH;
+#pragma unroll
+      for (int t = 0; t < AT; ++t) {
+        float* d = acc[j][t][0];
+#pragma unroll
+        for (int c = 1; c < CH; ++c)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) d[e] += acc[j][t][c][e];
+        if (F == 16) {     // a lane has features fr and fr + 8 of rows 2 kl and 2 kl + 1
+          float* r = r0 + t * 8 * FW_RED_PITCH;
+          r[(2 * kl) * FW_RED_PITCH + fr] = d[0];
+          r[(2 * kl + 1) * FW_RED_PITCH + fr] = d[1];
+          r[(2 * kl) * FW_RED_PITCH + fr + 8] = d[2];
+          r[(2 * kl + 1) * FW_RED_PITCH + fr + 8] = d[3];
+        } else {           // features 2 kl and 2 kl + 1 of rows fr and fr + 8
+          *reinterpret_cast<float2*>(r0 + fr * FW_RED_PITCH + 2 * kl) = make_float2(d[0], d[1]);
+          *reinterpret_cast<float2*>(r0 + (fr + 8) * FW_RED_PITCH + 2 * kl) = make_float2(d[2], d[3]);
+        }
+      }
+    }
+    __syncthreads();
+    if (S > 1 && warp == 0 && g + S < groups) ask(g + S, slot);   // every warp has read this group's weights
+#pragma unroll
+    for (int q = 0; q < OUTS; ++q) {
+      int j, m, nl;
+      const bool ok = place(q, j, m, nl) && g * GT + j < mine;
+      const int n = (t_begin + g * GT + j) * F + nl;
+      if (!ok || n >= N) continue;
+      float p[FW_WARPS];
+#pragma unroll
+      for (int w = 0; w < FW_WARPS; ++w) p[w] = rd[((w * GT + j) * ROWS + m) * FW_RED_PITCH + nl];
+      float x = ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7])) + bias_r[q];
+      if (prm.act == ACT_GELU_TANH) {
+        float th;
+        asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(0.7978845608028654f * (x + 0.044715f * x * x * x)));
+        x = 0.5f * x * (1.0f + th);
+      } else if (prm.act == ACT_GELU_ERF) {
+        x = gelu_erf(x);
+      } else if (prm.act == ACT_RELU_SQ) {
+        x = relu_sq(x);
+      }
+      if (kv_at[q] != -1) {
+        if (kv_at[q] == -3)
+          *prm.status = NIB_STATUS_BAD_PAGE;
+        else if (kv_at[q] >= 0)
+          prm.kv_cache[kv_at[q]] = __float2bfloat16_rn(x);
+      } else if (prm.out_f32) {
+        ((float*)prm.out)[(size_t)(row0 + m) * prm.ldo + n] = prm.residual ? res_r[q] + x : x;
+      } else {
+        ((bf16*)prm.out)[(size_t)(row0 + m) * prm.ldo + n] = __float2bfloat16_rn(x);
+      }
+    }
+    if (++slot == S) { slot = 0; ++round; }
+  }
+  if (abort_sh) {   // a copy did not come in time: no thread leaves while one may still be under way
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      *prm.status = NIB_STATUS_WAIT_TIMEOUT;
+      const long long t0 = clock64();
+      for (int i = 0; i < S && i < groups; ++i)
+        while (!mbar_try_wait(&bars[i], ((groups - 1 - i) / S) & 1) && clock64() - t0 < TC_WAIT_CYCLES) {}
+    }
+    __syncthreads();
+  }
+}
+
+template <int F, int GT, int ST, bool LN>
+static int launch_few_rows_of(const FewParams& prm, const FewPlan& p, cudaStream_t stream) {
+  static const cudaError_t attr = cudaFuncSetAttribute(linear_few_rows_kernel<F, GT, ST, LN>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FW_SMEM_LIMIT);
+  if (attr != cudaSuccess) return (int)attr;
+  cudaError_t e = launch_pdl(linear_few_rows_kernel<F, GT, ST, LN>, dim3(p.blocks, p.row_blocks), dim3(FW_WARPS * 32), p.smem,
+                             stream, prm);
+  if (e != cudaSuccess) return (int)e;
+  NIB_LAUNCH_CHECK();
+}
+
+template <int F, int GT, bool LN>
+static int launch_few_rows_st(const FewParams& prm, const FewPlan& p, cudaStream_t stream) {
+  switch (p.ST) {
+    case 3: return launch_few_rows_of<F, GT, 3, LN>(prm, p, stream);
+    case 4: return launch_few_rows_of<F, GT, 4, LN>(prm, p, stream);
+    case 7: return launch_few_rows_of<F, GT, 7, LN>(prm, p, stream);
+  }
+  if constexpr (!LN && GT == 1) {
+    switch (p.ST) {
+      case 12: return launch_few_rows_of<F, GT, 12, LN>(prm, p, stream);
+      case 16: return launch_few_rows_of<F, GT, 16, LN>(prm, p, stream);
+      case 25: return launch_few_rows_of<F, GT, 25, LN>(prm, p, stream);
+    }
+  }
+  return NIB_ERR_UNSUPPORTED_SIZE;
+}
+
+int launch_few_rows(const FewParams& prm, const FewPlan& p, bool ln, cudaStream_t stream) {
+  if (p.F == 8) return launch_few_rows_st<8, 1, false>(prm, p, stream);
+  switch (p.GT) {
+    case 1: return ln ? launch_few_rows_st<16, 1, true>(prm, p, stream) : launch_few_rows_st<16, 1, false>(prm, p, stream);
+    case 2: return ln ? launch_few_rows_st<16, 2, true>(prm, p, stream) : launch_few_rows_st<16, 2, false>(prm, p, stream);
+    default: return ln ? launch_few_rows_st<16, 3, true>(prm, p, stream) : launch_few_rows_st<16, 3, false>(prm, p, stream);
+  }
+}
+
+
+}  // namespace nib

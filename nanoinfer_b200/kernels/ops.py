@@ -567,12 +567,36 @@ def linear_skinny(a, norm, w, bias, out, M, act=ACT_NONE, residual=False, kv=Non
     return True
 
 
-FEW_MAX_ROWS = 8
+FEW_MAX_ROWS = 128
+
+
+def few_pays(M: int, N: int, K: int, norm: bool) -> bool:
+    """Whether a product goes to the kernel for few rows (M <= 128) rather than to tcgen05, whose rows a norm of its own
+    normalises.  Up to 16 rows always.  Beyond, the step is cut into row blocks of 16 that share the 148 SMs, and what
+    counts is how many tiles of 16 features a block then has.  Measured in whole steps (us; this rule, all on this kernel,
+    none beyond 16 rows, and gemm_skinny.cu, which took most of these before):
+      small decode 32 rows 1568, 1567, 2355, 1915     61 rows 2099, 2099, 2584, 2239     prompt 77 464, 467, 516, 481
+      medium decode 24 rows 3195, 3192, 4761, 3760    61 rows 6557, 6689, 6958, 6730     prompt 77 992, 1194, 1074, 1130
+      XL decode 40 rows 12661, 12661, 14404, 14421    61 rows 14713, 15152, 15029, 15048   prompt 77 2813, 3137, 2817, 2832
+    The second MLP product reads rows of 3,072 and more values again for every tile, so one or two tiles a block; wide
+    outputs (the head) are tcgen05's from 17 rows on."""
+    if M <= 16:
+        return True
+    if M > FEW_MAX_ROWS or N > 8192:
+        return False
+    places, tiles = 148 // (-(-M // 16)), -(-N // 16)
+    most = -(-tiles // min(tiles, places))       # tiles that a block has
+    if K > 1792:
+        return most <= (2 if K <= 3072 else 1)
+    if norm:
+        return M <= (80 if K <= 768 else 64 if K <= 1024 else 48) and most <= (7 if K <= 1024 else 9)
+    return most <= 3
 
 
 def linear_few(a, norm, w, bias, out, M, act=ACT_NONE, residual=False, kv=None) -> bool:
-    """The kernel for steps of at most 8 rows (bfloat16): one block an SM, its weights by the copy engine into shared
-    memory, the rows from memory to the MMAs' registers.  Options as for ``linear_skinny``; False where it does not apply."""
+    """The kernel for steps of at most 128 rows (bfloat16) that makes up for few rows: one block an SM, its weights by the copy
+    engine into shared memory, the rows from memory to the MMAs' registers.  Options as for ``linear_skinny``; False where
+    it does not apply."""
     if M > FEW_MAX_ROWS or not _small_inputs_ok(a, norm, w, out):
         return False
     N, K = w.shape
@@ -613,36 +637,22 @@ def linear_small_tc(a, norm, w, bias, out, M, act=ACT_NONE, residual=False, kv=N
     return True
 
 
-def skinny_pays(M: int, N: int, K: int) -> bool:
-    """Whether a product of at most 128 rows goes to the warp-level MMA kernel rather than to tcgen05.
-    Measured in whole decode steps at widths 768, 1024 and 1600 (batch 16 to 64): up to 16 rows the MMA
-    kernel wins everywhere; up to 32 rows everywhere but the longest rows (K of 4096 and more, split over a
-    cluster: GPT-2 medium's second MLP product at 32 rows is 4 % of a step slower here, XL's 20 %) and the
-    widest outputs (the head), where its 16-feature tiles read the rows too often; beyond 32 rows while a row
-    block holds its rows unsplit.  Flipping one product's choice at a time at 24 to 128 rows and three widths
-    moves a step by less than 5 % where the other choice is better and by up to 97 % where it is worse.  (Alone, on
-    weights that the L2 holds, a norm and tcgen05 are ahead from 64 to 80 rows on, 10.6 against 12.5 us for 64 x 4096 x
-    1024; in a step, where the weights come from the memory, a prompt of 77 tokens takes 0.54 ms that way and 0.45 so.)"""
-    if M <= 16:
-        return True
-    if N > 8192 or M > SKINNY_MAX_ROWS:
-        return False
-    # (33 to 128 rows: while a row block holds its rows unsplit, K up to about a thousand.  The MLP's second
-    # product at GPT-2 medium's sizes, K = 4096, on tcgen05 instead: a decode step of 64 rows 1.17 against 1.37 ms)
-    return K <= (3072 if M <= 32 else 1088)
+def skinny_pays(M: int, kv) -> bool:
+    """Whether a product of at most 128 rows that the kernel for few rows does not take goes to gemm_skinny.cu rather than to
+    tcgen05: steps of up to 16 rows (sizes beyond that kernel's: K over 6,400, or a norm of more than 1,792 values), and, for
+    more, cache-writing projections whose heads tcgen05's epilogue does not take."""
+    return M <= 16 or (kv is not None and M <= SKINNY_MAX_ROWS and (kv[4] % 64 != 0 or kv[0].shape[4] % 16 != 0))
 
 
 def _linear_small(a, norm, w, bias, out, M, act, residual, kv=None) -> bool:
-    """Steps of at most 128 rows: the warp-level MMA kernel (with the LayerNorm folded in) where
-    ``skinny_pays``, else tcgen05.  Folding the norm into the tcgen05 kernel, or splitting
+    """Steps of at most 128 rows: the warp-level MMA kernels (with the LayerNorm folded in) where
+    ``few_pays`` or ``skinny_pays``, else tcgen05.  Folding the norm into the tcgen05 kernel, or splitting
     K through scratch, costs more round trips than it saves at these sizes, so that kernel is given
     normed rows and is not split here."""
     N, K = w.shape
-    # (up to 8 rows: measured ahead of the kernel for up to 128 rows at every product of widths 768, 1024 and 1600, see there)
-    if M <= FEW_MAX_ROWS and linear_few(a, norm, w, bias, out, M, act, residual, kv):
+    if few_pays(M, N, K, norm is not None) and linear_few(a, norm, w, bias, out, M, act, residual, kv):
         return True
-    mma = skinny_pays(M, N, K)
-    if mma:
+    if skinny_pays(M, kv):
         # (rows wider than SKINNY_LN_REGISTER_WIDTH are normalised through a buffer per warp in shared memory, which
         # leaves room for one block an SM from 9 rows on: GPT-2 XL at batch 12 to 32 is 2 to 7 % faster with the
         # norm as a kernel of its own there)

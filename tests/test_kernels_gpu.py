@@ -810,12 +810,15 @@ def test_few_row_product_with_k_split_over_a_cluster(M, N, K, split):
 # a ring of several; steps of K: one piece, a ragged step, the edges between the kernels' numbers of steps
 FEW_SHAPES = [(1, 7, 8, False), (8, 1184, 768, False), (3, 1185, 776, False), (8, 16, 24, True), (1, 2369, 768, True),
               (8, 4737, 1024, True), (5, 7105, 1032, True), (2, 7200, 1792, True), (8, 9001, 256, False), (8, 768, 3072, False),
-              (7, 1000, 4096, False), (4, 1600, 6400, False), (8, 17, 1600, False)]
+              (7, 1000, 4096, False), (4, 1600, 6400, False), (8, 17, 1600, False),
+              # row blocks of sixteen: one, one row more, a ragged last one, the most; few places a row block
+              (9, 1184, 768, False), (16, 2369, 1600, True), (17, 40, 3072, False), (61, 3072, 1024, True), (128, 600, 264, True),
+              (40, 1600, 4096, False), (33, 9, 8, False)]
 
 
 @pytest.mark.parametrize("M, N, K, ln", FEW_SHAPES)
-def test_product_of_at_most_eight_rows(M, N, K, ln):
-    """The kernel for 1 to 8 rows against 64 bits: its epilogues, a norm with and without shift, rows by a list, what lies
+def test_product_of_few_rows(M, N, K, ln):
+    """The kernel for 1 to 128 rows against 64 bits: its epilogues, a norm with and without shift, rows by a list, what lies
     beside the result untouched.  Products of bfloat16 are exact in 32 bits, so a 32-bit output is off by the additions'
     rounding at most; a normalised row may round the other way at a tie, half a unit of bfloat16's last place (2^-8) a value."""
     o = ops()
@@ -864,7 +867,8 @@ def test_product_of_at_most_eight_rows(M, N, K, ln):
             alone = torch.zeros(1, N, device=DEV)
             one = None if norm is None else o.NormInput(norm.x, norm.gamma, norm.beta, 1e-5, ws, torch.bfloat16, rows=norm.rows[M - 1:].contiguous())
             assert o.linear_few(None if norm is not None else ad[M - 1:], one, wd, bd, alone, 1)
-            assert torch.equal(alone[0], buf[M - 1, :N])
+            # (beyond eight rows tiles may be grouped in another way, and the chains of a sum with them)
+            assert torch.equal(alone[0], buf[M - 1, :N]) if M <= 8 else ((alone[0].cpu().double() - got[M - 1, :N]).abs() <= 2 * bound[M - 1]).all()
     assert int(o.status_word().item()) == 0
 
 
