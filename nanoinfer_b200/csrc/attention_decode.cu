@@ -159,10 +159,13 @@ attention_decode_kernel(const T* q, int ldq, const T* cache, float* part_o,
       }
     }
   };
+  const float inv_cap = ex.softcap > 0.0f ? 1.0f / ex.softcap : 0.0f;
   // none of the first batch's keys is the one that the kernel ahead writes
   const bool early = n_kept > 0 || (n_main > 0 && (first_batch + warp) * BK + BK - 1 < pos);
   if (early) fetch(0);
   pdl_wait();
+  // a head's gate, asked for with the query (at the end it would be a round trip of its own)
+  const float gate_r = ex.gate && ex.gate_dim == 0 ? ex.gate[(size_t)t * ex.ldg + h] : 0.0f;
   if (cluster_merge) cluster_wait();   // every block of the cluster runs by now
 
   if (empty) {
@@ -212,7 +215,7 @@ attention_decode_kernel(const T* q, int ldq, const T* cache, float* part_o,
         sc[b] = ((live >> b) & 1u) ? dot * scale2 : -INFINITY;
       } else {
         float sv = dot * scale;
-        if (ex.softcap > 0.0f) sv = ex.softcap * tanhf(sv / ex.softcap);
+        if (ex.softcap > 0.0f) sv = ex.softcap * tanhf(sv * inv_cap);
         sv -= slope * (float)(pos - (cur_j0 + b * GROUPS + group));
         sc[b] = ((live >> b) & 1u) ? sv * 1.4426950408889634f : -INFINITY;
       }
@@ -250,17 +253,25 @@ attention_decode_kernel(const T* q, int ldq, const T* cache, float* part_o,
       *reinterpret_cast<float4*>(go + g * head_dim + c * VN + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);
   }
   __syncthreads();
-  float M = -INFINITY;
-  for (int w = 0; w < ALL_GROUPS; ++w) M = fmaxf(M, gm[w]);
+  // (every thread makes every group's weight once; a group without a key has none)
+  float M = -INFINITY, share[ALL_GROUPS];
+#pragma unroll
+  for (int w = 0; w < ALL_GROUPS; ++w) share[w] = gm[w];
+#pragma unroll
+  for (int w = 0; w < ALL_GROUPS; ++w) M = fmaxf(M, share[w]);
   float L = 0.0f;
-  for (int w = 0; w < ALL_GROUPS; ++w) L += (gm[w] == -INFINITY) ? 0.0f : gl[w] * pow2<T>(gm[w] - M);
+#pragma unroll
+  for (int w = 0; w < ALL_GROUPS; ++w) share[w] = share[w] == -INFINITY ? 0.0f : pow2<T>(share[w] - M);
+#pragma unroll
+  for (int w = 0; w < ALL_GROUPS; ++w) L += gl[w] * share[w];
   // a sink (one more term in the denominator: a key of score 0 without a value) counts once, where the row's
   // weights are divided
   const float L1 = (sink && n_splits == 1) ? L + pow2<T>(sink2 - M) : L;
-  const float mul1 = n_splits == 1 ? ex.out_scale * (ex.gate && ex.gate_dim == 0 ? 1.0f / (1.0f + expf(-ex.gate[(size_t)t * ex.ldg + h])) : 1.0f) : 1.0f;
+  const float mul1 = n_splits == 1 ? ex.out_scale * (ex.gate && ex.gate_dim == 0 ? 1.0f / (1.0f + expf(-gate_r)) : 1.0f) : 1.0f;
   for (int d = threadIdx.x; d < head_dim; d += blockDim.x) {
     float acc = 0.0f;
-    for (int w = 0; w < ALL_GROUPS; ++w) acc += (gm[w] == -INFINITY) ? 0.0f : go[w * head_dim + d] * pow2<T>(gm[w] - M);
+#pragma unroll
+    for (int w = 0; w < ALL_GROUPS; ++w) acc = fmaf(go[w * head_dim + d], share[w], acc);
     if (n_splits == 1) {
       const float y = acc / L1 * mul1 * element_gate(ex, t, h, d);
       if (ex.out32) reinterpret_cast<float*>(out)[(size_t)t * ldo + h * head_dim + d] = y;
@@ -303,18 +314,41 @@ attention_decode_kernel(const T* q, int ldq, const T* cache, float* part_o,
     if (!is_last_sh) return;
     __threadfence();
   }
-  float Mx = -INFINITY;
-  for (int sp = 0; sp < n_splits; ++sp) Mx = fmaxf(Mx, part_ml[2 * (base + sp)]);
-  float Lx = 0.0f;
-  for (int sp = 0; sp < n_splits; ++sp) {
-    const float ls = part_ml[2 * (base + sp) + 1];
-    if (ls > 0.0f) Lx += ls * pow2<T>(part_ml[2 * (base + sp)] - Mx);
+  // Up to eight splits: all loads at once, their weights 2^(m - max) in registers; more: a walk for each
+  constexpr int FEW = 8;
+  float Mx = -INFINITY, Lx = 0.0f, ms[FEW], ls8[FEW];
+  const bool few = n_splits <= FEW;
+  if (few) {
+#pragma unroll
+    for (int sp = 0; sp < FEW; ++sp) {
+      ms[sp] = sp < n_splits ? part_ml[2 * (base + sp)] : -INFINITY;
+      ls8[sp] = sp < n_splits ? part_ml[2 * (base + sp) + 1] : 0.0f;
+    }
+#pragma unroll
+    for (int sp = 0; sp < FEW; ++sp) Mx = fmaxf(Mx, ms[sp]);
+#pragma unroll
+    for (int sp = 0; sp < FEW; ++sp) {
+      ms[sp] = ls8[sp] > 0.0f ? pow2<T>(ms[sp] - Mx) : 0.0f;
+      Lx += ls8[sp] * ms[sp];
+    }
+  } else {
+    for (int sp = 0; sp < n_splits; ++sp) Mx = fmaxf(Mx, part_ml[2 * (base + sp)]);
+    for (int sp = 0; sp < n_splits; ++sp) {
+      const float ls = part_ml[2 * (base + sp) + 1];
+      if (ls > 0.0f) Lx += ls * pow2<T>(part_ml[2 * (base + sp)] - Mx);
+    }
   }
   if (sink) Lx += pow2<T>(sink2 - Mx);
-  const float mulx = ex.out_scale * (ex.gate && ex.gate_dim == 0 ? 1.0f / (1.0f + expf(-ex.gate[(size_t)t * ex.ldg + h])) : 1.0f);
+  const float mulx = ex.out_scale * (ex.gate && ex.gate_dim == 0 ? 1.0f / (1.0f + expf(-gate_r)) : 1.0f);
   for (int d = threadIdx.x; d < head_dim; d += blockDim.x) {
     float acc = 0.0f;
-    for (int sp = 0; sp < n_splits; ++sp) {
+    if (few) {
+      float v[FEW];      // (a split without a key left nothing to read)
+#pragma unroll
+      for (int sp = 0; sp < FEW; ++sp) v[sp] = ls8[sp] > 0.0f ? part_o[(base + sp) * head_dim + d] : 0.0f;
+#pragma unroll
+      for (int sp = 0; sp < FEW; ++sp) acc = fmaf(v[sp], ms[sp], acc);
+    } else for (int sp = 0; sp < n_splits; ++sp) {
       const float ls = part_ml[2 * (base + sp) + 1];
       if (ls > 0.0f) acc += part_o[(base + sp) * head_dim + d] * pow2<T>(part_ml[2 * (base + sp)] - Mx);
     }
@@ -332,9 +366,10 @@ static int launch_decode(const void* q, int ldq, const void* cache, float* part_
                          int n_splits, int* counters, int* status, cudaStream_t stream) {
   dim3 grid(n_splits, n_head, n_rows);
   const int n_pieces = head_dim / Piece<T>::N;
-  // two or four splits run as one cluster and merge through distributed shared memory (clusters of
-  // eight measured slower than the merge through global scratch: they are harder to place)
-  const int cluster = (n_splits == 2 || n_splits == 4) ? n_splits : 1;
+  // Two to four splits run as one cluster and merge through distributed shared memory, up to eight where all clusters
+  // stand at once with a block an SM (a decode step of one row over a window of 512 keys, 12 heads in 8 splits: with the
+  // merge's loads at once 11.4 -> 7.4 us a launch; larger grids of eight are harder to place and were slower).
+  const int cluster = n_splits >= 2 && (n_splits <= 4 || (n_splits <= 8 && (long long)n_rows * n_head * n_splits <= 148)) ? n_splits : 1;
 #define NIB_DECODE_LAUNCH(LPR)                                                                                     \
   launch_pdl_cluster(attention_decode_kernel<T, LPR>, dim3(grid), dim3(DEC_WARPS * 32),                            \
              (size_t)(DEC_WARPS * (32 / LPR) * (head_dim + 2) + n_splits * (head_dim + 2)) * sizeof(float), stream, \
