@@ -826,7 +826,11 @@ def test_product_of_few_rows(M, N, K, ln):
     g = gen(M + N + K)
     a = torch.randn(M + 2, K, generator=g).to(torch.bfloat16)
     w, b = (torch.randn(N, K, generator=g) * 0.05).to(torch.bfloat16), torch.randn(N, generator=g)
-    wd, bd, ad = w.to(DEV), b.to(DEV), a.to(DEV)
+    # (rows of a wider buffer: the kernel takes any pitch that is a multiple of eight)
+    wide_w, wide_a = torch.zeros(N, K + 8, dtype=torch.bfloat16, device=DEV), torch.zeros(M + 2, K + 16, dtype=torch.bfloat16, device=DEV)
+    wd, ad, bd = wide_w[:, :K], wide_a[:, :K], b.to(DEV)
+    wd.copy_(w)
+    ad.copy_(a)
     norms = [None]
     if ln:
         x = torch.randn(M + 2, K, generator=g) * 1.5 - 0.3
